@@ -391,8 +391,8 @@ CUWHHD_API wp_status wp_sweep2d_solve(float* qz, const float* xv, const float* y
 
 /* Allocation-free DST-I Poisson solve.  No reference counterpart (CuDst3D allocates its buffers in
    its constructor).  Same result as wp_dst3d_create + wp_dst3d_solve, but no handle and no device
-   allocation on any call: the three DST-I matrices and the intermediate buffer live in one static
-   device array of 3*64*64 + 64^3 doubles (2.2 MB) inside the library.  For callers that cannot
+   allocation on any call: the three DST-I matrices live in one static device array of 3*64*64
+   doubles (98 KB) inside the library.  For callers that cannot
    allocate: a solver running under a fixed device-memory budget whose pool is already committed,
    or a stream-ordered loop next to other streams where cudaFree's implicit device synchronization
    would stall them.

@@ -205,3 +205,23 @@ def test_dirichlet_sweep_and_mid_sweep_reproduce_fields_at_64(wp):
         c = fields.curl3d(*[t.double().cpu().numpy() for t in q], (n, n, n), (h, h, h))
         assert np.sqrt(sum(np.sum((a - b) ** 2) for a, b in zip(u, c)) / den) < 1e-5, (bc, mid)
         sw.close()
+
+
+@pytest.mark.parametrize("n", [(1, 2, 3), (7, 16, 9), (17, 33, 31), (32, 15, 255), (256, 5, 4), (4, 257, 3), (3, 2, 512),
+                               (513, 3, 2), (2, 1024, 17)])
+def test_dst3d_tile_edges_match_oracle(wp, oracle, n):
+    """Extents around the kernel's tiles (16 outputs, 8 inputs, 32 or 16 lines, the three line-length
+    classes), out of place and in place.  Bound: two FP64 transforms per axis, each a sum of at most N
+    terms with orthonormal weights, plus the table's rounding: 6 N eps of the result."""
+    h = tuple(1.0 / (v + 1) for v in n)
+    f = np.random.default_rng(sum(n)).standard_normal((n[2], n[0], n[1]))
+    ref = oracle.dst3d_poisson(f, n, h)
+    ft = torch.as_tensor(f, dtype=torch.float64, device="cuda")
+    out = torch.full_like(ft, float("nan"))
+    solver = wp.CuDst3D(n, h)
+    solver.Solve(out, ft)
+    solver.Solve(ft, ft)
+    torch.cuda.synchronize()
+    bound = 6 * (max(n) + 8) * 2.3e-16
+    assert _rel(ref, out.cpu().numpy()) < bound
+    assert torch.equal(out, ft)
