@@ -114,3 +114,11 @@ cudaError_t wp_set_smem(K kernel, size_t bytes) {
 template <typename T>
 wp_status wp_dwt_axis_launch(T* dst, const T* src, int DX, int DY, int DZ, int levels, char axis, int wavelet,
                              char bc, int forward, cudaStream_t stream);
+// up to three FP32 passes along one axis (equal levels), in one launch where they can be
+struct WpDwtPass {
+    float* dst;
+    const float* src;
+    int DX, DY, DZ, wavelet;
+    char bc;
+};
+wp_status wp_dwt_axis_launch_n(const WpDwtPass* q, int n, int levels, char axis, int forward, cudaStream_t stream);

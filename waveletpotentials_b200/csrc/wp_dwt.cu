@@ -729,6 +729,300 @@ __global__ void __launch_bounds__(NT) dwt_tile_kernel(const T* __restrict__ src,
     }
 }
 
+// ---- CDF3.7 and CDF4.6 on lines of up to 512 (+ 1) samples: in place on one tile of 32 lines.
+//
+// What bounded dwt_tile_kernel there was issue: 89 instructions a sample (windows of 16 pairs read for 8,
+// signs and reflection tables on every pair, staging through registers), 71 to 83 us for a pass over 256^3
+// whose bytes take 20 (now 42 to 47, and 40 with three components in a launch).  Here a warp's lanes are 32 lines and its registers hold the window of P pairs (P = 16
+// at the top level) with their halo; a level reads its windows, synchronises, and writes back to the same
+// tile, which halves the shared memory and leaves the Mallat layout in place.  The ends of a line are P-pair
+// windows like the others whose outer four pairs are read at constant reflected offsets.  Samples arrive
+// by cp.async, all of a CTA's in flight at once; along x and z the details (forward) and the last level
+// (inverse) go from registers to memory.  Up to three arrays of the same axis share a launch.
+// Measured (B200): recovery of 256 x 128 x 64, 18 passes, 293 -> 125 us; FP64 CDF4.6 of 8300 lines of 257 samples
+// 24.6 -> 18.4 us.
+struct LineJob {
+    const void* src;
+    void* dst;
+    long s_in, s_out, pstride; // between lines, between outer indices, along the line
+    int ni, lines;             // lines per outer index, lines in all
+    int N, levels, bcd, c4;    // c4: CDF4.6, else CDF3.7
+};
+struct LineJobs {
+    LineJob j[3];
+};
+constexpr int kLineCP = 33;
+
+__device__ __forceinline__ void cp_async_sample(float* d, const float* s) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(s) : "memory");
+}
+__device__ __forceinline__ void cp_async_sample(double* d, const double* s) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(s) : "memory");
+}
+
+// One chunk of P pairs [k0, k0 + P) of a level with nd details (and nd + C4 approximations): the window's pair
+// w is pair k0 - 4 + w.  E: even samples or approximations, O: odd samples or details, x(i) and y(i) their
+// readers; sg: the sign of a reflected value ('d' walls).
+template <typename T, bool C4, bool FWD, int P>
+struct Chunk {
+    T A[P + 8], D[P + 8];
+    T sl, sr; // signs of the D (and A) values left and right of the line (inverse CDF4.6: undone after each step)
+
+    __device__ __forceinline__ void read(const T* X, int k0, int nd, int bcd) {
+        constexpr int CP = kLineCP;
+        const bool first = k0 == 0, last = k0 + P == nd;
+        const T sg = bcd ? T(-1) : T(1);
+        sl = sr = T(1);
+        if (FWD) {
+            const T* b = X + 2 * k0 * CP;
+#pragma unroll
+            for (int w = 4; w < P + 4; ++w) {
+                A[w] = b[(2 * w - 8) * CP];
+                D[w] = b[(2 * w - 7) * CP];
+            }
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                // pair -4 + w: sample -i is sample i (CDF4.6) or i - 1 (CDF3.7)
+                constexpr int h = C4 ? 0 : 1;
+                A[w] = first ? sg * b[(8 - 2 * w - h) * CP] : b[(2 * w - 8) * CP];
+                D[w] = first ? sg * b[(7 - 2 * w - h) * CP] : b[(2 * w - 7) * CP];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                // pair nd + t: sample 2 nd + i is sample 2 nd - i (CDF4.6, whose sample 2 nd exists) or 2 nd - 1 - i
+                constexpr int h = C4 ? 0 : 1;
+                const int w = P + 4 + t;
+                A[w] = last ? (C4 && t == 0 ? T(1) : sg) * b[(2 * P - 2 * t - h) * CP] : b[(2 * w - 8) * CP];
+                D[w] = last ? sg * b[(2 * P - 1 - 2 * t - h) * CP] : b[(2 * w - 7) * CP];
+            }
+        } else {
+            const T* a = X + k0 * CP;
+            const T* d = X + (nd + (C4 ? 1 : 0) + k0) * CP;
+            // reflected details change sign where approximations do (CDF4.6) or where they do not (CDF3.7)
+            const T sd = C4 ? sg : -sg;
+            if (first) sl = sg;
+            if (last) sr = sg;
+#pragma unroll
+            for (int w = 4; w < P + 4; ++w) {
+                A[w] = a[(w - 4) * CP];
+                D[w] = d[(w - 4) * CP];
+            }
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                A[w] = first ? sg * a[(C4 ? 4 - w : 3 - w) * CP] : a[(w - 4) * CP];
+                D[w] = first ? sd * d[(3 - w) * CP] : d[(w - 4) * CP];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int w = P + 4 + t;
+                A[w] = last ? (C4 && t == 0 ? T(1) : sg) * a[(C4 ? P - t : P - 1 - t) * CP] : a[(w - 4) * CP];
+                D[w] = last ? sd * d[(P - 1 - t) * CP] : d[(w - 4) * CP];
+            }
+        }
+    }
+
+    // afterwards A[4 + j], D[4 + j] are output pair k0 + j (A also at j = P, CDF4.6's last approximation or sample)
+    __device__ __forceinline__ void lift() {
+        constexpr int W = P + 8;
+        if (FWD && !C4) {
+#pragma unroll
+            for (int w = W - 1; w >= 1; --w) A[w] += T(K37::fu1) * D[w - 1];
+#pragma unroll
+            for (int w = 1; w < W - 1; ++w) D[w] = D[w] + T(K37::fp0) * A[w + 1] + T(K37::fp1) * A[w];
+            using K = K3<WP_ID_CDF3_7>;
+#pragma unroll
+            for (int w = 4; w < P + 4; ++w)
+                A[w] = (A[w] + T(K::q6) * D[w - 3] + T(K::q5) * D[w - 2] + T(K::q4) * D[w - 1] + T(K::q3) * D[w] +
+                        T(K::q2) * D[w + 1] + T(K::q1) * D[w + 2] + T(K::q0) * D[w + 3]) * T(K37::scl0);
+#pragma unroll
+            for (int w = 4; w < P + 4; ++w) D[w] *= T(K37::scl1);
+        } else if (FWD) {
+#pragma unroll
+            for (int w = W - 1; w >= 1; --w) A[w] = A[w] + T(K46::fu1_1) * D[w - 1] + T(K46::fu1_0) * D[w];
+#pragma unroll
+            for (int w = 1; w < W - 1; ++w) D[w] = D[w] + T(K46::fp1) * A[w] + T(K46::fp0) * A[w + 1];
+#pragma unroll
+            for (int w = 4; w <= P + 4; ++w)
+                A[w] = (A[w] + T(K46::c5) * D[w - 3] + T(K46::c4) * D[w - 2] + T(K46::c3) * D[w - 1] + T(K46::c2) * D[w] +
+                        T(K46::c1) * D[w + 1] + T(K46::c0) * D[w + 2]) * T(K46::scl0);
+#pragma unroll
+            for (int w = 4; w < P + 4; ++w) D[w] *= T(K46::scl1);
+        } else if (!C4) {
+            using K = K3<WP_ID_CDF3_7>;
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                A[w] *= T(K37::scl1);
+                D[w] *= T(K37::scl0);
+            }
+#pragma unroll
+            for (int w = 3; w < P + 5; ++w)
+                A[w] -= T(K::q6) * D[w - 3] + T(K::q5) * D[w - 2] + T(K::q4) * D[w - 1] + T(K::q3) * D[w] +
+                        T(K::q2) * D[w + 1] + T(K::q1) * D[w + 2] + T(K::q0) * D[w + 3];
+#pragma unroll
+            for (int w = 3; w < P + 4; ++w) D[w] -= T(K37::fp1) * A[w] + T(K37::fp0) * A[w + 1];
+#pragma unroll
+            for (int w = 4; w < P + 4; ++w) A[w] -= T(K37::fu1) * D[w - 1];
+        } else {
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                D[w] *= T(K46::scli1);
+                A[w] *= T(K46::scli0);
+            }
+            // dwt_tile_kernel multiplies reflected values by their sign after each step: both forms' outputs are
+            // the same reads with the sign moved from the update to the value it corrects
+#pragma unroll
+            for (int w = 3; w < P + 6; ++w) {
+                const T u = T(K46::c5) * D[w - 3] + T(K46::c4) * D[w - 2] + T(K46::c3) * D[w - 1] + T(K46::c2) * D[w] +
+                            T(K46::c1) * D[w + 1] + T(K46::c0) * D[w + 2];
+                A[w] -= u;
+                if (w < 4) A[w] *= sl;
+                if (w > P + 4) A[w] *= sr;
+            }
+            // D = SD D, then D = SD (D - predict): a reflected detail keeps its value and loses SD x the predict
+#pragma unroll
+            for (int w = 3; w < P + 5; ++w) {
+                const T pr = T(K46::fp1) * A[w] + T(K46::fp0) * A[w + 1];
+                D[w] -= w < 4 ? sl * pr : w >= P + 4 ? sr * pr : pr;
+            }
+#pragma unroll
+            for (int w = 4; w <= P + 4; ++w) A[w] -= T(K46::fu1_1) * D[w - 1] + T(K46::fu1_0) * D[w];
+        }
+    }
+};
+
+// One level of the tile: forward from the interleaved samples X[0, 2 nd + ext) to approximations X[0, nd + ext)
+// and details behind them, inverse the other way.  DIRECT: the details (forward) or all samples (inverse) go
+// to g (position 0 of this thread's line, step ps; null: no line) instead of the tile.
+template <typename T, bool C4, bool FWD, int P, bool DIRECT>
+__device__ __forceinline__ void line_level(T* X, T* g, long ps, int warp, int nd, int bcd) {
+    constexpr int CP = kLineCP, X1 = C4 ? 1 : 0;
+    const int k0 = warp * P;
+    const bool on = k0 < nd, last = k0 + P == nd;
+    Chunk<T, C4, FWD, P> c;
+    if (on) {
+        c.read(X, k0, nd, bcd);
+        c.lift();
+    }
+    if (!(DIRECT && !FWD)) __syncthreads();
+    if (on) {
+        if (FWD) {
+            T* a = X + k0 * CP;
+#pragma unroll
+            for (int j = 0; j < P; ++j) a[j * CP] = c.A[4 + j];
+            if (C4 && last) a[P * CP] = c.A[4 + P];
+            if (DIRECT) {
+                if (g) {
+                    T* d = g + (long)(nd + X1 + k0) * ps;
+#pragma unroll
+                    for (int j = 0; j < P; ++j, d += ps) *d = c.D[4 + j];
+                }
+            } else {
+                T* d = X + (nd + X1 + k0) * CP;
+#pragma unroll
+                for (int j = 0; j < P; ++j) d[j * CP] = c.D[4 + j];
+            }
+        } else if (DIRECT) {
+            if (g) {
+                T* d = g + (long)(2 * k0) * ps;
+#pragma unroll
+                for (int j = 0; j < P; ++j) {
+                    *d = c.A[4 + j];
+                    d += ps;
+                    *d = c.D[4 + j];
+                    d += ps;
+                }
+                if (C4 && last) *d = c.A[4 + P];
+            }
+        } else {
+            T* d = X + 2 * k0 * CP;
+#pragma unroll
+            for (int j = 0; j < P; ++j) {
+                d[2 * j * CP] = c.A[4 + j];
+                d[(2 * j + 1) * CP] = c.D[4 + j];
+            }
+            if (C4 && last) d[2 * P * CP] = c.A[4 + P];
+        }
+    }
+    if (!(DIRECT && !FWD)) __syncthreads();
+}
+
+// P0: pairs per warp at the top level (the CTA has 2^(levels - 1) / P0 warps)
+template <typename T, bool C4, bool FWD, bool DIRECT, int P0>
+__device__ __forceinline__ void line_run(T* X, T* g, long ps, const LineJob& J, int warp, int lane) {
+    constexpr int NB = C4 ? 5 : 4;
+    const double* mat = C4 ? c_base46[(FWD ? 0 : 2) + J.bcd] : c_base37[(FWD ? 0 : 2) + J.bcd];
+    if (FWD) {
+        const int top = 1 << (J.levels - 1), nw = blockDim.x >> 5;
+        for (int nd = top; nd >= 4; nd >>= 1) {
+            if (P0 > 8 && nd >= P0 * nw) line_level<T, C4, true, P0, DIRECT>(X, g, ps, warp, nd, J.bcd);
+            else if (nd >= 8) line_level<T, C4, true, 8, DIRECT>(X, g, ps, warp, nd, J.bcd);
+            else line_level<T, C4, true, 4, DIRECT>(X, g, ps, warp, nd, J.bcd);
+        }
+        if (warp == 0) {
+            base_level_n<T, NB>(mat, X, X, kLineCP);
+            if (DIRECT && g)
+                for (int p = 0; p < NB; ++p) g[p * ps] = X[p * kLineCP];
+        }
+        if (!DIRECT) __syncthreads();
+    } else {
+        if (warp == 0) base_level_n<T, NB>(mat, X, X, kLineCP);
+        __syncthreads();
+        const int top = 1 << (J.levels - 1), nw = blockDim.x >> 5;
+        for (int nd = 4; nd < top; nd <<= 1) {
+            if (nd >= 8) line_level<T, C4, false, 8, false>(X, g, ps, warp, nd, J.bcd);
+            else line_level<T, C4, false, 4, false>(X, g, ps, warp, nd, J.bcd);
+        }
+        if (top < 4) {  // N = 4 (+ 1): the base level alone
+            if (DIRECT && g && warp == 0)
+                for (int p = 0; p < NB; ++p) g[p * ps] = X[p * kLineCP];
+        } else if (P0 > 8 && top >= P0 * nw) {
+            line_level<T, C4, false, P0, DIRECT>(X, g, ps, warp, top, J.bcd);
+        } else if (top >= 8) {
+            line_level<T, C4, false, 8, DIRECT>(X, g, ps, warp, top, J.bcd);
+        } else {
+            line_level<T, C4, false, 4, DIRECT>(X, g, ps, warp, top, J.bcd);
+        }
+    }
+}
+
+template <typename T, bool FWD, bool CONTIG, int P0, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) dwt_line_kernel(const __grid_constant__ LineJobs jobs) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    wp_pdl_enter();
+    const LineJob& J = jobs.j[blockIdx.y];
+    const int l0 = blockIdx.x * 32;
+    if (l0 >= J.lines) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, N = J.N;
+    T* sm = reinterpret_cast<T*>(smem_raw);
+    const T* src = static_cast<const T*>(J.src);
+    T* dst = static_cast<T*>(J.dst);
+    T* X = sm + lane;
+    T* g = nullptr;
+    if (CONTIG) {
+        // a warp per line, lanes along it
+        for (int c = warp; c < 32 && l0 + c < J.lines; c += nw) {
+            const T* line = src + (long)(l0 + c) * J.s_in;
+            for (int p = lane; p < N; p += 32) cp_async_sample(sm + p * kLineCP + c, line + p);
+        }
+    } else if (l0 + lane < J.lines) {
+        const int o = (l0 + lane) / J.ni, i = l0 + lane - o * J.ni;
+        const long at = o * J.s_out + i * J.s_in;
+        g = dst + at;
+        const T* q = src + at + warp * J.pstride;
+        for (int p = warp; p < N; p += nw, q += nw * J.pstride) cp_async_sample(X + p * kLineCP, q);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (J.c4) line_run<T, true, FWD, !CONTIG, P0>(X, g, J.pstride, J, warp, lane);
+    else line_run<T, false, FWD, !CONTIG, P0>(X, g, J.pstride, J, warp, lane);
+    if (CONTIG) {
+        for (int c = warp; c < 32 && l0 + c < J.lines; c += nw) {
+            T* line = dst + (long)(l0 + c) * J.s_in;
+            for (int p = lane; p < N; p += 32) line[p] = sm[p * kLineCP + c];
+        }
+    }
+}
+
 bool g_const_ready[64] = {false};
 std::mutex g_const_mu;
 
@@ -830,13 +1124,66 @@ cudaError_t launch_c(const T* src, T* dst, int N, int levels, int bcd, TileGeom 
     }
 }
 
-}  // namespace
-
+// Whether dwt_line_kernel takes the pass: its windows hold lines of up to 512 samples in FP32 (16 warps of 16
+// pairs, 128 registers a thread) and 256 in FP64 (16 warps of 8); longer lines would need more warps than the
+// registers allow, so they, and the other wavelets, stay with dwt_tile_kernel.  CDF3.7 lines of 2^L + 1 and
+// CDF4.6 lines of 2^L samples stay there as well.
 template <typename T>
-wp_status wp_dwt_axis_launch(T* dst, const T* src, int DX, int DY, int DZ, int levels, char axis, int wavelet,
-                             char bc, int forward, cudaStream_t stream) {
+bool line_ok(int wavelet, int N) {
+    const int ext = N & 1;
+    return N - ext <= (sizeof(T) == 4 ? 512 : 256) && (ext ? wavelet == WP_ID_CDF4_6 : wavelet == WP_ID_CDF3_7);
+}
+
+template <typename T, bool FWD, bool CONTIG, int P0, int MAXT, int MINB>
+cudaError_t launch_line_k(const LineJobs& jobs, dim3 grid, int nt, size_t smem, cudaStream_t s) {
+    auto kern = dwt_line_kernel<T, FWD, CONTIG, P0, MAXT, MINB>;
+    cudaError_t e = wp_set_smem(kern, smem);
+    if (e != cudaSuccess) return e;
+    wp_launch_pdl(kern, grid, nt, smem, s, jobs);
+    return cudaGetLastError();
+}
+
+// n passes along one axis (equal levels) in one launch
+template <typename T>
+cudaError_t launch_lines(const LineJobs& jobs, int n, bool contig, bool fwd, cudaStream_t s) {
+    constexpr int P0 = sizeof(T) == 4 ? 16 : 8;
+    const int top = 1 << (jobs.j[0].levels - 1), nt = 32 * std::max(1, top / P0);
+    int lines = 0, N = 0;
+    double bytes = 0;
+    for (int k = 0; k < n; ++k) {
+        lines = std::max(lines, jobs.j[k].lines);
+        N = std::max(N, jobs.j[k].N);
+        bytes += 2.0 * sizeof(T) * jobs.j[k].N * (double)jobs.j[k].lines;
+    }
+    const dim3 grid(wp_cdiv(lines, 32), n);
+    const size_t smem = sizeof(T) * (size_t)N * kLineCP;
+    const int tok = wp_prof_start(s);
+    cudaError_t e;
+    if constexpr (sizeof(T) == 4) {
+        if (nt <= 256)
+            e = fwd ? (contig ? launch_line_k<T, true, true, P0, 256, 3>(jobs, grid, nt, smem, s)
+                              : launch_line_k<T, true, false, P0, 256, 3>(jobs, grid, nt, smem, s))
+                    : (contig ? launch_line_k<T, false, true, P0, 256, 3>(jobs, grid, nt, smem, s)
+                              : launch_line_k<T, false, false, P0, 256, 3>(jobs, grid, nt, smem, s));
+        else
+            e = fwd ? (contig ? launch_line_k<T, true, true, P0, 512, 1>(jobs, grid, nt, smem, s)
+                              : launch_line_k<T, true, false, P0, 512, 1>(jobs, grid, nt, smem, s))
+                    : (contig ? launch_line_k<T, false, true, P0, 512, 1>(jobs, grid, nt, smem, s)
+                              : launch_line_k<T, false, false, P0, 512, 1>(jobs, grid, nt, smem, s));
+    } else {
+        e = fwd ? (contig ? launch_line_k<T, true, true, P0, 512, 1>(jobs, grid, nt, smem, s)
+                          : launch_line_k<T, true, false, P0, 512, 1>(jobs, grid, nt, smem, s))
+                : (contig ? launch_line_k<T, false, true, P0, 512, 1>(jobs, grid, nt, smem, s)
+                          : launch_line_k<T, false, false, P0, 512, 1>(jobs, grid, nt, smem, s));
+    }
+    wp_prof_stop(tok, fwd ? "dwt_forward" : "dwt_inverse", bytes, s);
+    return e;
+}
+
+// checks a pass and sets its geometry, lines, outer extent and wall rule (0 'n', 1 'd', 2 'z')
+wp_status dwt_plan(const void* dst, int DX, int DY, int DZ, int levels, char axis, int wavelet, char bc, TileGeom& g, int& N,
+                   int& nouter, int& bcd) {
     if (!dst || DX <= 0 || DY <= 0 || DZ <= 0) { wp_set_error_msg("wp_dwt1d: bad arguments"); return WP_ERR_INVALID_ARG; }
-    if (!src) src = dst;
     const bool shortf = wavelet == WP_ID_CDF2_0 || is_t1(wavelet);
     if (!is_q3(wavelet) && !is_c4(wavelet) && !is_l2(wavelet) && !shortf) {
         wp_set_error_msg("wp_dwt1d: wavelet must be CDF3.5, CDF3.7, CDF4.4, CDF4.6, CDF2.6, CDF2.8, CDF2.0, "
@@ -852,8 +1199,6 @@ wp_status wp_dwt_axis_launch(T* dst, const T* src, int DX, int DY, int DZ, int l
     // CDF2.x have a rule of their own (:802-828, 928-933)
     if (bc == 'z' && !is_l2(wavelet)) bc = is_q3(wavelet) ? 'd' : 'n';
     if (bc != 'n' && bc != 'd' && bc != 'z') { wp_set_error_msg("wp_dwt1d: bc must be 'n', 'd' or 'z'"); return WP_ERR_INVALID_ARG; }
-    TileGeom g;
-    int N, nouter;
     switch (axis) {
         case 'y': case 'Y': N = DY; g.s_in = DY; g.ni = DX; g.s_out = (long)DX * DY; nouter = DZ; g.pstride = 1; g.contiguous = 1; break;
         case 'x': case 'X': N = DX; g.s_in = 1; g.ni = DY; g.s_out = (long)DX * DY; nouter = DZ; g.pstride = DY; g.contiguous = 0; break;
@@ -866,7 +1211,6 @@ wp_status wp_dwt_axis_launch(T* dst, const T* src, int DX, int DY, int DZ, int l
         return WP_ERR_INVALID_ARG;
     }
     if (nouter > 65535) { wp_set_error_msg("wp_dwt1d: outer extent too large"); return WP_ERR_UNSUPPORTED; }
-    WP_CUDA_TRY(ensure_constants());
     if ((wavelet == WP_ID_CDF4_4 || l2_rules(wavelet)) && !(N & 1)) {
         // their base matrices act on five coefficients: whole-sample lines of 2^levels + 1
         wp_set_error_msg("wp_dwt1d: CDF4.4 and CDF2.x lines have 2^levels + 1 samples");
@@ -877,9 +1221,30 @@ wp_status wp_dwt_axis_launch(T* dst, const T* src, int DX, int DY, int DZ, int l
         wp_set_error_msg("wp_dwt1d: CDF1.x lines have 2^levels samples");
         return WP_ERR_INVALID_ARG;
     }
-    const int bcd = bc == 'd' ? 1 : (bc == 'z' ? 2 : 0);
+    bcd = bc == 'd' ? 1 : (bc == 'z' ? 2 : 0);
+    WP_CUDA_TRY(ensure_constants());
+    return WP_OK;
+}
+
+LineJob line_job(const void* src, void* dst, const TileGeom& g, int N, int nouter, int levels, int bcd, int wavelet) {
+    return LineJob{src, dst, g.s_in, g.s_out, g.pstride, g.ni, g.ni * nouter, N, levels, bcd, wavelet == WP_ID_CDF4_6};
+}
+
+}  // namespace
+
+template <typename T>
+wp_status wp_dwt_axis_launch(T* dst, const T* src, int DX, int DY, int DZ, int levels, char axis, int wavelet,
+                             char bc, int forward, cudaStream_t stream) {
+    TileGeom g;
+    int N, nouter, bcd;
+    wp_status st = dwt_plan(dst, DX, DY, DZ, levels, axis, wavelet, bc, g, N, nouter, bcd);
+    if (st != WP_OK) return st;
+    if (!src) src = dst;
     cudaError_t e;
-    if (wavelet == WP_ID_CDF3_7)
+    if (line_ok<T>(wavelet, N) && (double)g.ni * nouter < 2e9) {
+        const LineJobs jobs{{line_job(src, dst, g, N, nouter, levels, bcd, wavelet)}};
+        e = launch_lines<T>(jobs, 1, g.contiguous != 0, forward != 0, stream);
+    } else if (wavelet == WP_ID_CDF3_7)
         e = forward ? launch_c<WP_ID_CDF3_7, true, T>(src, dst, N, levels, bcd, g, nouter, stream)
                     : launch_c<WP_ID_CDF3_7, false, T>(src, dst, N, levels, bcd, g, nouter, stream);
     else if (wavelet == WP_ID_CDF3_5)
@@ -910,6 +1275,33 @@ wp_status wp_dwt_axis_launch(T* dst, const T* src, int DX, int DY, int DZ, int l
     return WP_OK;
 }
 
+// up to three passes along one axis, in one launch where dwt_line_kernel takes them all
+wp_status wp_dwt_axis_launch_n(const WpDwtPass* q, int n, int levels, char axis, int forward, cudaStream_t stream) {
+    LineJobs jobs{};
+    bool one = true;
+    int contig = 0;
+    for (int k = 0; k < n; ++k) {
+        TileGeom g;
+        int N, nouter, bcd;
+        wp_status st = dwt_plan(q[k].dst, q[k].DX, q[k].DY, q[k].DZ, levels, axis, q[k].wavelet, q[k].bc, g, N, nouter, bcd);
+        if (st != WP_OK) return st;
+        one = one && line_ok<float>(q[k].wavelet, N) && (double)g.ni * nouter < 2e9;
+        contig = g.contiguous;
+        jobs.j[k] = line_job(q[k].src, q[k].dst, g, N, nouter, levels, bcd, q[k].wavelet);
+    }
+    if (one) {
+        cudaError_t e = launch_lines<float>(jobs, n, contig != 0, forward != 0, stream);
+        if (e != cudaSuccess) { wp_set_cuda_error(e, "dwt launch", __FILE__, __LINE__); return WP_ERR_CUDA; }
+        return WP_OK;
+    }
+    for (int k = 0; k < n; ++k) {
+        wp_status st = wp_dwt_axis_launch<float>(q[k].dst, q[k].src, q[k].DX, q[k].DY, q[k].DZ, levels, axis, q[k].wavelet,
+                                                 q[k].bc, forward, stream);
+        if (st != WP_OK) return st;
+    }
+    return WP_OK;
+}
+
 // Times the pass over the tile widths 4..32 that fit shared memory (median of three single launches,
 // in place on buf) and records the fastest for this shape.  Synchronous; buf's contents are
 // overwritten.
@@ -917,6 +1309,7 @@ template <typename T>
 wp_status wp_dwt_axis_tune(T* buf, int DX, int DY, int DZ, int levels, char axis, int wavelet, char bc, int forward,
                            cudaStream_t s) {
     const int N = (axis == 'y' || axis == 'Y') ? DY : (axis == 'x' || axis == 'X') ? DX : DZ;
+    if (line_ok<T>(wavelet, N)) return WP_OK;  // dwt_line_kernel has one tile width
     cudaEvent_t a, b;
     WP_CUDA_TRY(cudaEventCreate(&a));
     WP_CUDA_TRY(cudaEventCreate(&b));
