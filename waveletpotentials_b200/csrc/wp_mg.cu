@@ -1837,12 +1837,7 @@ __device__ __forceinline__ void lean_cycle(const LPack& P, int nu1, int nu2, flo
     for (int i = tid; i < S[0].cells; i += B) out[i] = v0[i];
 }
 
-__global__ void __launch_bounds__(1024) coarse_cycle_lean_kernel(LPack P, int nu1, int nu2, float w, int citers,
-                                                                 int prolong) {
-    wp_pdl_enter();
-    extern __shared__ __align__(16) float lean_smem[];
-    lean_cycle(P, nu1, nu2, w, citers, prolong, lean_smem);
-}
+#include "wp_mg_cluster.cuh"
 
 // ---- persistent cycle below the finest level --------------------------------------------------
 // Levels 1 .. k of a V-cycle are small (at 256^3: 128^3, 64^3, 32^3), L2-resident and latency bound:
@@ -2698,7 +2693,7 @@ struct wp_mgfrac3d {
     int coarsest_iters;
     double* acc;       // device reduction slots; then the int error flag (acc + 4) and the grid
                        // barrier words of mid_cycle_kernel (8 bytes further)
-    int mid_on;        // run the levels below the finest as one persistent launch (autotuned, default on)
+    int mid_on;        // run the levels below the finest as one persistent launch (autotuned, default off)
     int mid_forbid;    // never (handles whose cycles share the GPU with concurrent graph branches)
     int mid_grid;      // its CTAs (one per SM; 0 = not yet known, -1 = not possible on this device)
     double* p64;       // FP64 iterate for mixed precision
@@ -2717,6 +2712,9 @@ struct wp_mgfrac3d {
     int loop_key[7];   // nu1, nu2, prolongation, full-multigrid first cycle, tune_gen, device, inner cycles
     double loop_omega;
     long long loop_launches[2]; // kernels of the first cycle's graph part and of one loop body
+    CyPlan cy;         // the small levels' single-launch cycle (FP32): its levels are cy.l0 .. nl - 1
+    int cy_from;       // levels above this one run their own kernels (wp_mgfrac3d_set_tile pins a level)
+    CyPlan cy1;        // a handle that shares the device: the levels of the pack that one CTA holds
     int fz_on;         // run the V(2,2) FP32 cycle of level 0 as the two fused kernels where it fits
     int fz_zc;         // their z planes per CTA (0 = heuristic)
     int ix_built;      // the index lists of every level exist
@@ -2863,6 +2861,80 @@ wp_status build_hierarchy(wp_mgfrac3d* h, const float* ax, const float* ay, cons
         }
     }
     return WP_OK;
+}
+
+template <bool D2>
+cudaError_t cy_prepare() {
+    cudaError_t e = wp_set_smem(cycle_cluster_kernel<D2>, kCySmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(cycle_cluster_kernel<D2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+
+// The pack of small levels: the finest level from which all the rest fits the shared memory of up to `most`
+// CTAs (a cluster of 16 needs the non-portable size; B200 places it on one GPC).  With 16, cubes from 32^3
+// and 2D grids from 256^2; a cycle from there takes 31 and 50 us, where launches took 75 (from 32^3) and 110.
+wp_status build_cycle_plan(wp_mgfrac3d* h, CyPlan* q, int most, cudaStream_t s) {
+    const bool d2 = h->dims == 2;
+    q->l0 = h->nl;
+    for (int l = 0; l + 2 <= h->nl; ++l) {
+        int e[kMaxLevels][3];
+        for (int k = l; k < h->nl; ++k) {
+            const int* n = h->lv[k].n;
+            e[k - l][0] = d2 ? 1 : n[0];
+            e[k - l][1] = n[1];
+            e[k - l][2] = d2 ? n[0] : n[2];
+        }
+        int ctas = most;
+        while (ctas > 1 && ctas / 2 >= e[0][2]) ctas /= 2;
+        if (cy_layout(&q->pack, e, h->nl - l, ctas, d2)) {
+            q->l0 = l;
+            break;
+        }
+    }
+    if (q->l0 == h->nl) return WP_OK;
+    WP_CUDA_TRY(d2 ? cy_prepare<true>() : cy_prepare<false>());
+    WP_CUDA_TRY(cudaMalloc((void**)&q->image, sizeof(float) * (size_t)q->pack.image * q->pack.ctas));
+    WP_CUDA_TRY(cudaMemsetAsync(q->image, 0, sizeof(float) * (size_t)q->pack.image * q->pack.ctas, s));
+    for (int k = 0; k < q->pack.n; ++k) {
+        const Level& L = h->lv[q->l0 + k];
+        const dim3 g(std::min<unsigned>(wp_cdiv(q->pack.lv[k].cap, 256), 64), q->pack.ctas);
+        WP_KERNEL("cycle_coeff", 40.0 * L.cells, s,
+                  (d2 ? cy_coeff_kernel<true><<<g, 256, 0, s>>>(q->image, q->pack, k, view<float>(L))
+                      : cy_coeff_kernel<false><<<g, 256, 0, s>>>(q->image, q->pack, k, view<float>(L))));
+    }
+    return WP_OK;
+}
+
+// the cycle from level l of the pack (see cycle_cluster_kernel)
+cudaError_t launch_cycle_cluster(const wp_mgfrac3d* h, const CyPlan& q, int l, const float* f, const float* vin, float* vout,
+                                 double* p64, int nu1, int nu2, float w, int prolong, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(q.pack.ctas);
+    cfg.blockDim = dim3(kCyThreads);
+    cfg.dynamicSmemBytes = sizeof(float) * (size_t)q.pack.floats;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = q.pack.ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = s == nullptr || s == cudaStreamLegacy || s == cudaStreamPerThread ? 1 : 2;
+    auto k = h->dims == 2 ? cycle_cluster_kernel<true> : cycle_cluster_kernel<false>;
+    return cudaLaunchKernelEx(&cfg, k, q.pack, (const float*)q.image, l - q.l0, f, vin, vout, p64, nu1, nu2, w,
+                              h->coarsest_iters, prolong);
+}
+
+// n sweeps of level l of the pack by its global-memory kernel (zero: from zero); the result is in L.v
+template <bool D2>
+void launch_cy_sweeps(Level& L, const CyGlobal& G, const float* f, int n, float w, bool zero, cudaStream_t s) {
+    for (int k = 0; k < n; ++k) {
+        wp_launch_pdl(cy_sweep_kernel<D2>, wp_cdiv(G.n, 256), 256, 0, s, L.t, (const float*)(zero && k == 0 ? nullptr : L.v), f,
+                      G, w);
+        std::swap(L.v, L.t);
+    }
 }
 
 wp_status ensure_fp64(wp_mgfrac3d* h) {
@@ -3064,6 +3136,8 @@ wp_status coarsest_solve(wp_mgfrac3d* h, Level& L, const T* f, T w, cudaStream_t
     return smooth<T>(L, f, h->coarsest_iters, w, s);
 }
 
+wp_status cy_level(wp_mgfrac3d* h, int l, const float* f, int nu1, int nu2, float w, int prolong, cudaStream_t s, bool clear_v);
+
 // One V-cycle at level l from the level's current v, or (clear_v) from v = 0: then v is neither
 // cleared nor read -- the first sweep is jacobi0_q_kernel where the level's kernel allows, otherwise
 // v is cleared first -- and below kCoarseCells the single-launch coarse cycle takes over.
@@ -3081,33 +3155,25 @@ wp_status vcycle(wp_mgfrac3d* h, int l, const T* f, int nu1, int nu2, T w, int p
             if (done) return WP_OK;
         }
     }
+    if constexpr (sizeof(T) == 4) {
+        if (l >= h->cy.l0 && l >= h->cy_from && l < h->nl - 1) {
+            if (h->cy1.image && l < h->cy1.l0) return cy_level(h, l, f, nu1, nu2, (float)w, prolong, s, clear_v);
+            // the rest of the cycle in one launch of one cluster
+            const CyPlan& q = h->cy1.image ? h->cy1 : h->cy;
+            double* acc = added ? acc64 : nullptr;
+            cudaError_t e = cudaSuccess;
+            WP_KERNEL("coarse_cycle", (double)L.cells * (3.0 * sizeof(T) + 12.0) * (nu1 + nu2 + 2), s,
+                      e = launch_cycle_cluster(h, q, l, f, clear_v ? nullptr : L.v, L.v, acc, nu1, nu2, (float)w, prolong, s));
+            if (e != cudaSuccess) { wp_set_cuda_error(e, "cycle cluster", __FILE__, __LINE__); return WP_ERR_CUDA; }
+            if (acc) *added = true;
+            return WP_OK;
+        }
+    }
     long pack_cells = 0;
     for (int k = l; k < h->nl; ++k) pack_cells += h->lv[k].cells;
     if (clear_v && l > 0 && l < h->nl - 1 && L.cells <= kCoarseCells && h->nl - l <= kCoarseMax &&
         f == Bufs<T>::f(L) && pack_cells <= kCoarseSmemCells) {
         // the rest of the cycle in one launch; the host mirrors the buffer swaps it performs
-        bool lean = sizeof(T) == 4;
-        LPack Q;
-        Q.n = h->nl - l;
-        for (int k = 0; k < Q.n && lean; ++k) {
-            Level& E = h->lv[l + k];
-            lean = E.ccf != nullptr;
-            Q.lv[k] = {E.n[0], E.n[1], E.n[2], E.ccf, (float*)Bufs<T>::v(E), (float*)Bufs<T>::t(E),
-                       (const float*)Bufs<T>::f(E)};
-        }
-        const size_t lean_bytes = lean ? sizeof(float) * (size_t)lean_smem_floats(Q) : 0;
-        if (lean && lean_bytes <= kLeanSmemMax) {
-            WP_CUDA_TRY(wp_set_smem(coarse_cycle_lean_kernel, kLeanSmemMax));
-            WP_KERNEL("coarse_cycle", (double)L.cells * (3.0 * sizeof(T) + 12.0) * (nu1 + nu2 + 2), s,
-                      wp_launch_pdl(coarse_cycle_lean_kernel, 1, 1024, lean_bytes, s, Q, nu1, nu2, (float)w,
-                                    h->coarsest_iters, prolong));
-            for (int k = 0; k < Q.n; ++k) {
-                Level& E = h->lv[l + k];
-                const int swaps = (k == Q.n - 1) ? h->coarsest_iters : nu1 + nu2;
-                if (swaps & 1) std::swap(Bufs<T>::v(E), Bufs<T>::t(E));
-            }
-            return WP_OK;
-        }
         const size_t smem_max = 3 * sizeof(T) * (size_t)kCoarseSmemCells;
         WP_CUDA_TRY(wp_set_smem(coarse_cycle_kernel<T>, smem_max));
         CPack<T> P;
@@ -3330,6 +3396,8 @@ void destroy_levels(wp_mgfrac3d* h) {
         for (void* p : ps) if (p) cudaFree(p);
     }
     if (h->ccf_all) cudaFree(h->ccf_all);
+    for (CyPlan* q : {&h->cy, &h->cy1})
+        if (q->image) cudaFree(q->image);
     if (h->acc) cudaFree(h->acc);
     if (h->p64) cudaFree(h->p64);
     if (h->r32) cudaFree(h->r32);
@@ -3351,9 +3419,10 @@ wp_status create_common(wp_mgfrac3d** out, int dims, const float* ax, const floa
     if (!h) return WP_ERR_INVALID_ARG;
     h->dims = dims;
     h->coarsest_iters = dims == 3 ? 50 : 10;
-    h->mid_on = 1;
+    h->mid_on = 0;
     h->fz_on = 1;
     wp_status st = build_hierarchy(h, ax, ay, az, nx, ny, nz, dx, dy, dz, s);
+    if (st == WP_OK) st = build_cycle_plan(h, &h->cy, 16, s);
     if (st == WP_OK) {
         cudaError_t e = cudaMalloc((void**)&h->acc, 4 * sizeof(double) + 16);
         // the int error flag lives in the 16 bytes after the four FP64 slots
@@ -3444,6 +3513,32 @@ wp_status build_index(wp_mgfrac3d* h, cudaStream_t s) {
     if (dev) cudaFree(dev);
     if (st == WP_OK) h->ix_built = 1;
     return st;
+}
+
+// The cycle from level l of the pack, level l launch by launch (the cluster's arithmetic, see cy_cell)
+wp_status cy_level(wp_mgfrac3d* h, int l, const float* f, int nu1, int nu2, float w, int prolong, cudaStream_t s, bool clear_v) {
+    Level &L = h->lv[l], &C = h->lv[l + 1];
+    const CyPack& P = h->cy.pack;
+    const CyLev &a = P.lv[l - h->cy.l0], &c = P.lv[l + 1 - h->cy.l0];
+    const CyGlobal G{h->cy.image + a.cf, P.image, a.cap, a.nx, a.ny, a.nz, a.nxy, (int)L.cells};
+    const bool d2 = h->dims == 2;
+    auto sweeps = [&](int n, float wt, bool zero) {
+        if (d2) launch_cy_sweeps<true>(L, G, f, n, wt, zero, s);
+        else launch_cy_sweeps<false>(L, G, f, n, wt, zero, s);
+    };
+    const double bytes = (double)L.cells * 4.0 * cy_floats(d2);
+    WP_KERNEL("jacobi_shared", (bytes + 12.0 * L.cells) * std::max(nu1, 1), s,
+              (clear_v && nu1 == 0 ? sweeps(1, 0.f, true) : sweeps(nu1, w, clear_v)));
+    WP_KERNEL("resid_restrict_shared", bytes + 8.0 * L.cells + 4.0 * C.cells, s,
+              wp_launch_pdl(d2 ? cy_restrict_kernel<true> : cy_restrict_kernel<false>, wp_cdiv(C.cells, 256), 256, 0, s, C.f,
+                            (const float*)L.v, f, G, c.nx, c.ny, (int)C.cells));
+    const wp_status st = vcycle<float>(h, l + 1, C.f, nu1, nu2, w, prolong, s, true);
+    if (st != WP_OK) return st;
+    WP_KERNEL("prolong_shared", 8.0 * L.cells + 4.0 * C.cells, s,
+              wp_launch_pdl(d2 ? cy_prolong_kernel<true> : cy_prolong_kernel<false>, wp_cdiv(L.cells, 256), 256, 0, s, L.v,
+                            (const float*)C.v, G, c.nx, c.ny, c.nz, prolong));
+    WP_KERNEL("jacobi_shared", (bytes + 12.0 * L.cells) * nu2, s, sweeps(nu2, w, false));
+    return WP_OK;
 }
 
 // One index-sparse V-cycle at level l (SolveOneVCycle_index, cuMultigridFrac3D.cu:366-420).  A
@@ -4918,7 +5013,9 @@ wp_status autotune(wp_mgfrac3d* h, cudaStream_t s) {
         cudaMemsetAsync(L.v, 0, sizeof(float) * L.cells, s);
         cudaMemsetAsync(L.f, 0, sizeof(float) * L.cells, s);
         const int kinds = (l == 0 && h->p64 && h->r32) ? 3 : (l + 1 < h->nl ? 2 : 1);
-        for (int kind = 0; kind < kinds; ++kind) {
+        // the pack's levels run no sweep or restriction of their own
+        const bool packed = l >= h->cy.l0 && l >= h->cy_from;
+        for (int kind = packed ? kZcDefect : 0; kind < kinds; ++kind) {
             const auto key = std::make_tuple(dev, kind, nx, ny, nz);
             {
                 std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -4979,7 +5076,7 @@ wp_status autotune(wp_mgfrac3d* h, cudaStream_t s) {
     }
     // the levels below the finest as one persistent launch, or launch by launch: time a V-cycle from
     // level 1 both ways (the levels are L2-resident: no flush) and keep the faster
-    if (st == WP_OK && h->dims == 3 && h->nl >= 3 && !h->mid_forbid) {
+    if (st == WP_OK && h->dims == 3 && h->nl >= 3 && !h->mid_forbid && h->cy.l0 > 1) {
         float best = 1e30f;
         int best_on = 1;
         for (int on = 1; on >= 0 && st == WP_OK; --on) {
@@ -5000,7 +5097,7 @@ wp_status autotune(wp_mgfrac3d* h, cudaStream_t s) {
     // adds into an FP64 iterate -- here a scratch array, not the handle's), after an L2 flush when
     // level 0 exceeds it; the fused passes only when they are clearly (5%) faster -- at 256^3 the
     // two measure alike and the one-sweep kernels use the memory bandwidth better per byte
-    if (st == WP_OK && h->dims == 3 && h->nl >= 2 && h->lv[0].tuni) {
+    if (st == WP_OK && h->dims == 3 && h->nl >= 2 && h->lv[0].tuni && h->cy.l0 > 0) {
         Level& L0 = h->lv[0];
         double* acc = nullptr;
         if (cudaMalloc((void**)&acc, sizeof(double) * L0.cells) != cudaSuccess) {
@@ -5073,6 +5170,7 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_set_tile(wp_mgfrac3d* h, int level, 
         // level 0's V(2,2) cycle: the two fused kernels (1) or one kernel per sweep / transfer (0)
         h->fz_on = variant;
         h->fz_zc = zc > 0 ? zc + (zc & 1) : 0;
+        h->cy_from = std::max(h->cy_from, 1);  // a pinned level runs its own kernels
         ++h->tune_gen;
         return WP_OK;
     }
@@ -5085,6 +5183,7 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_set_tile(wp_mgfrac3d* h, int level, 
     L.zc[kind] = zc > 0 ? zc : 0;
     L.var[kind] = variant;
     L.zc_ms[kind] = 0.f;
+    if (kind != kZcDefect) h->cy_from = std::max(h->cy_from, level + 1);  // a pinned level runs its own kernels
     ++h->tune_gen;
     return WP_OK;
 }
@@ -5102,9 +5201,19 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_uniform_rows(const wp_mgfrac3d* h, i
 }
 
 wp_status wp_mg_prepare_mixed(wp_mgfrac3d* h) { return prepare_mixed(h); }
-// a cooperative launch needs the whole GPU: the batch, whose grids run on concurrent graph branches,
-// keeps every level launch by launch
-void wp_mg_forbid_persistent(wp_mgfrac3d* h) { h->mid_forbid = 1; }
+// For the batch, whose grids run on concurrent graph branches.  A cooperative launch needs the whole GPU, so
+// the levels go launch by launch, and of the pack only those that one CTA holds share a launch: a cluster of 16
+// is faster for one grid and dearer for many (16 SMs for 31 to 50 us a cycle: 64 uneven 2D and 3D grids took
+// 31.4 ms with it, 28.6 before).  The pack's larger levels keep its arithmetic, so that a grid's results are those
+// of its own solver; a pack whose last level is divided among the CTAs is kept whole.
+wp_status wp_mg_share_device(wp_mgfrac3d* h) {
+    h->mid_forbid = 1;
+    if (h->cy.l0 == h->nl || h->cy.pack.lv[h->cy.pack.n - 1].P != 0) return WP_OK;
+    const wp_status st = build_cycle_plan(h, &h->cy1, 1, nullptr);
+    if (st != WP_OK) return st;
+    WP_CUDA_TRY(cudaStreamSynchronize(nullptr));
+    return WP_OK;
+}
 wp_status wp_mg_solve_mixed_loop_capture(wp_mgfrac3d* h, float* dst, const float* f, const wp_mg_params* prm,
                                          cudaStream_t s, long long* body_launches) {
     return solve_mixed_loop_capture(h, dst, f, prm, s, body_launches);
