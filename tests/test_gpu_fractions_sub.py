@@ -48,3 +48,34 @@ def test_subsampled_fractions_match_oracle_at_64(wp, oracle):
         d = np.abs(o - r)
         assert d.max() <= 3 * SAMPLE and np.count_nonzero(d) <= max(3, r.size // 10000), d.max()
         assert np.all((o >= 0) & (o <= 1))
+
+
+@pytest.mark.parametrize("slope", [(1.0, 0.0, 0.0), (0.0, -0.5, 0.0), (0.0, 0.0, 1.0), (1.0, 0.25, -0.5), (0.5, 0.5, 0.5)])
+@pytest.mark.parametrize("n", [(5, 9, 7), (8, 33, 6)])
+@pytest.mark.parametrize("offset", [0.0, 1.0 / 1024, 5.0 / 32])
+def test_plane_fractions_are_exact_counts(wp, oracle, n, offset, slope):
+    """Planes with dyadic coefficients, the zero set on sample positions and cell centres.  Every product of
+    the interpolation is a dyadic number of fewer than 53 bits, so the sample values are exact and the counts
+    must be equal (bound 0).  In the first half cell the position is clamped to a number that is not dyadic: a
+    plane through its samples (offset 0) is left out there."""
+    h = 1.0 / 16
+    z, x, y = np.meshgrid(*[np.arange(k) + 0.5 for k in (n[2], n[0], n[1])], indexing="ij")
+    ls = (slope[0] * (x - n[0] / 2) + slope[1] * (y - n[1] / 2) + slope[2] * (z - n[2] / 2) + offset) * h
+    assert np.array_equal(ls, ls.astype(np.float32))
+    got = _frac(wp, ls.astype(np.float32), n, h)
+    at = (slice(1, None),) * 3 if offset == 0 else ()
+    for r, o in zip(oracle.fractions3d_subsampled(ls, n, h), got):
+        assert np.array_equal(o[at], r[at])
+
+
+def test_non_finite_level_sets_match_oracle(wp, oracle):
+    """A value that is not finite makes every face whose 27 taps hold it compare false (closed), taps of
+    weight 0 included.  No bound: comparisons only."""
+    n, h = (6, 40, 5), 1.0 / 16
+    ls = np.full((n[2], n[0], n[1]), 3 * h, dtype=np.float32)
+    ls[2, 3, 7] = np.nan
+    ls[2, 3, 20] = np.inf
+    ls[2, 3, 33] = -np.inf
+    for r, o in zip(oracle.fractions3d_subsampled(ls.astype(np.float64), n, h), _frac(wp, ls, n, h)):
+        assert np.array_equal(o, r)
+        assert (r == 0).any() and (r == 1).any()

@@ -460,6 +460,7 @@ extern "C" CUWHHD_API wp_status wp_recover3d_create(wp_recover3d** out, int nx, 
 
 extern "C" CUWHHD_API wp_status wp_recover3d_destroy(wp_recover3d* h) {
     if (!h) return WP_OK;
+    wp_scratch_trim();
     for (int a = 0; a < 3; ++a) {
         if (h->tab[a]) cudaFree(h->tab[a]);
         if (h->tmp[a]) cudaFree(h->tmp[a]);

@@ -27,6 +27,55 @@ int wp_sm_count() {
     return sms;
 }
 
+// Stream-ordered scratch from a memory pool of the library's own, one per device, that keeps up to
+// kScratchKeep bytes between calls (the default pool returns everything to the driver at the next
+// synchronisation, and the next allocation then costs about a millisecond).  What is above that goes back as
+// before, the rest when a solver or transform handle is destroyed (wp_scratch_trim); freed with cudaFreeAsync.  Thread- and stream-safe as the runtime's pools are.  A
+// stream that is being captured keeps the default pool (the allocation becomes a node of the graph).
+#include <mutex>
+
+namespace {
+constexpr unsigned long long kScratchKeep = 64ull << 20;
+std::mutex g_scratch_mu;
+cudaMemPool_t g_scratch_pool[64] = {nullptr};
+}  // namespace
+
+cudaError_t wp_scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &cs);
+    if (e != cudaSuccess) return e;
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if (cs != cudaStreamCaptureStatusNone || dev < 0 || dev >= 64) return cudaMallocAsync(p, bytes, s);
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lk(g_scratch_mu);
+        if (!g_scratch_pool[dev]) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
+            unsigned long long keep = kScratchKeep;
+            if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+                cudaMemPoolDestroy(pool);
+                return e;
+            }
+            g_scratch_pool[dev] = pool;
+        }
+        pool = g_scratch_pool[dev];
+    }
+    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
+// gives the current device's unused scratch back to the driver
+void wp_scratch_trim() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    if (g_scratch_pool[dev]) cudaMemPoolTrimTo(g_scratch_pool[dev], 0);
+}
+
 extern "C" CUWHHD_API const char* wp_last_error(void) { return g_err; }
 
 extern "C" CUWHHD_API int wp_version(void) { return 1; }
