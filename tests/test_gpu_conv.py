@@ -91,3 +91,19 @@ def test_conv3_rejects_bad_channels(wp):
     out = torch.zeros((2, 4, 4, 16), dtype=torch.bfloat16, device="cuda")
     with pytest.raises(wp.WPError):
         wp.conv3_forward(out, x, w)
+
+
+@pytest.mark.parametrize("n,cins,cout", [((201, 16, 16), (16,), 16), ((302, 4, 64), (32,), 32), ((331, 8, 32), (16, 64), 16),
+                                         ((5, 128, 128), (16,), 16), ((1, 4, 4), (32, 16), 64), ((3, 1, 2), (16,), 32)])
+def test_conv3_forward_columns_of_planes(wp, oracle, n, cins, cout):
+    """Columns of several planes per CTA with a shorter last one, tiles cut by the plane's end, weights of two
+    parts.  Bound: BF16 outputs, as above."""
+    rng = np.random.default_rng(sum(n) + cout)
+    xs = [oracle.bf16_round(rng.standard_normal(n + (c,))) for c in cins]
+    ws = [oracle.bf16_round(rng.standard_normal((27, cout, c)) / np.sqrt(27 * c)) for c in cins]
+    ref = sum(oracle.conv3d_forward(x, w) for x, w in zip(xs, ws))
+    out = torch.full(n + (cout,), float("nan"), dtype=torch.bfloat16, device="cuda")
+    kw = dict(x1=B(xs[1]), w1=B(ws[1])) if len(cins) > 1 else {}
+    wp.conv3_forward(out, B(xs[0]), B(ws[0]), **kw)
+    torch.cuda.synchronize()
+    assert rel(ref, F(out)) < 5e-3

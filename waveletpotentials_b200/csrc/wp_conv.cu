@@ -25,6 +25,7 @@
 #include "wp_common.cuh"
 #include "wp_tc.cuh"
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -36,6 +37,8 @@ constexpr int kThreads = 192;
 constexpr int kStagesF = 4;
 constexpr int kSlotA = 16384;  // 128 rows x 64 channels x 2 B
 constexpr int kSlotB = 8192;   // 64 x 64 x 2 B
+constexpr int kWalkThreads = 320; // weights, MMA, 4 epilogue and 4 producer warps
+constexpr int kStagesWalk = 6;  // input planes of the walk kernel's ring at most
 constexpr int kStagesW = 3;
 constexpr int kSlotWA = 32768;  // 128 x 128 x 2 B
 constexpr int kSlotWB = 16384;  // 128 x 64 x 2 B
@@ -65,6 +68,32 @@ __device__ __forceinline__ void load_bf16_row(const __nv_bfloat16* src, float* v
 struct TileGeo {
     int yt, xt, nty, ntx;
 };
+
+// one voxel's outputs: bias, skip addend, mask, ReLU, BF16 store
+template <int COUT>
+__device__ __forceinline__ void store_voxel(float* acc, long v, __nv_bfloat16* __restrict__ out,
+                                            const float* __restrict__ bias, const __nv_bfloat16* __restrict__ addend,
+                                            const __nv_bfloat16* __restrict__ mask, int relu) {
+    if (bias)
+#pragma unroll
+        for (int c = 0; c < COUT; ++c) acc[c] += bias[c];
+    if (addend) {
+        float a2[COUT];
+        load_bf16_row(addend + v * COUT, a2, COUT);
+#pragma unroll
+        for (int c = 0; c < COUT; ++c) acc[c] += a2[c];
+    }
+    if (mask) {
+        float mk[COUT];
+        load_bf16_row(mask + v * COUT, mk, COUT);
+#pragma unroll
+        for (int c = 0; c < COUT; ++c) acc[c] = mk[c] > 0.f ? acc[c] : 0.f;
+    }
+    if (relu)
+#pragma unroll
+        for (int c = 0; c < COUT; ++c) acc[c] = fmaxf(acc[c], 0.f);
+    store_bf16_row(out + v * COUT, acc, COUT);
+}
 
 // After a pipeline wait gave up: waits (bounded) for the tile loads issued but never consumed, steps
 // [consumed, issued) of the ring of full barriers, so that no copy into this CTA's shared memory is
@@ -175,25 +204,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int x = x0 + xi, y = y0 + yi;
         if (ready && x < nx && y < ny) {
             const long v = ((long)z * nx + x) * ny + y;
-            if (bias)
-#pragma unroll
-                for (int c = 0; c < COUT; ++c) acc[c] += bias[c];
-            if (addend) {
-                float a2[COUT];
-                load_bf16_row(addend + v * COUT, a2, COUT);
-#pragma unroll
-                for (int c = 0; c < COUT; ++c) acc[c] += a2[c];
-            }
-            if (mask) {
-                float mk[COUT];
-                load_bf16_row(mask + v * COUT, mk, COUT);
-#pragma unroll
-                for (int c = 0; c < COUT; ++c) acc[c] = mk[c] > 0.f ? acc[c] : 0.f;
-            }
-            if (relu)
-#pragma unroll
-                for (int c = 0; c < COUT; ++c) acc[c] = fmaxf(acc[c], 0.f);
-            store_bf16_row(out + v * COUT, acc, COUT);
+            store_voxel<COUT>(acc, v, out, bias, addend, mask, relu);
         }
     }
     tc_fence_before();
@@ -202,6 +213,208 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem, NCOL);
+    }
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Forward / input-gradient kernel that walks the planes of a column of tiles.  conv3_fwd_kernel fetches the
+// shifted input once per tap, 27 times in all (250 MB through L2 for 16 channels at 64^3, 70 us); here a CTA
+// keeps the layer's weights and a ring of input planes resident, each plane's halo block fetched once and
+// used for three output planes, and the x and y offsets are taken by moving the operand's start address.
+// That needs rows at a fixed pitch in one run, so a block is stored without swizzle, one part per 8 channels
+// of 16-byte rows [x][y = -1 .. ny], and the 128 rows of a tile are 128 consecutive positions of the padded
+// plane index x (ny + 2) + y: a tap (dx, dy) is the run that starts dx (ny + 2) + dy rows later.  Positions
+// with y >= ny compute padding that is not stored (2 / (ny + 2) of the work).  The blocks arrive by
+// 16-byte cp.async from four producer warps (zero-filled outside the volume).  Two accumulators in TMEM: the
+// epilogue of a plane overlaps the next plane's products.
+// What bounds it is the rate of the products, some 140 cycles each of 128 x N x 16 whatever N is.  Measured at
+// 64^3 (B200): 16 -> 16 channels 70 -> 32 us, 32 -> 32 78 -> 60, 16 + 32 -> 16 123 -> 79; at 32^3 and 16^3 within
+// 2 us of conv3_fwd_kernel, mostly below it.
+struct WalkGeo {
+    int pitch;     // ny + 2
+    int rows;      // x rows of a block
+    int tiles;     // per plane
+    unsigned mpitch; // position / pitch = umulhi(position, mpitch)
+    int lbo;       // bytes between the 8-channel parts of a block (a multiple of 128)
+    int slot;      // bytes of a ring step (one input plane, all its channels)
+    int w1, wbytes; // offset of the second part's weights, bytes of all
+    int stages;    // 0: does not fit
+    int zc;        // output planes per CTA
+};
+
+// 16 bytes, of which `bytes` (0 or 16) are read and the rest zero
+__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// The products of one input plane and part: 9 taps of CIN channels.  One thread issues them, so that building a
+// descriptor (some forty dependent instructions, 220 cycles) cost more than its product: two are built and the
+// others are sums (the address is their low field, in 16 bytes).
+template <int COUT, int CIN>
+__device__ __forceinline__ void walk_taps(uint32_t acc, uint32_t a, uint32_t b, const WalkGeo& g, uint32_t idesc, bool first) {
+    const uint64_t da = smem_desc(a, g.lbo, 128, 0), db = smem_desc(b, 16, 16 * CIN, sw_code(2 * CIN));
+    const uint32_t step = (uint32_t)g.lbo >> 3;  // two 8-channel parts
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+#pragma unroll
+        for (int j = 0; j < CIN / 16; ++j)
+            umma_f16(acc, da + (uint32_t)((t / 3) * g.pitch + t % 3 + j * step), db + (uint32_t)(t * COUT * CIN / 8 + 2 * j), idesc,
+                     !first || (t | j) != 0);
+}
+
+template <int COUT>
+__global__ void __launch_bounds__(kWalkThreads, 1)
+    conv3_walk_kernel(const __nv_bfloat16* __restrict__ xin0, const __grid_constant__ CUtensorMap wm0,
+                      const __nv_bfloat16* __restrict__ xin1, const __grid_constant__ CUtensorMap wm1, int cin0,
+                      int cin1, int nparts, __nv_bfloat16* __restrict__ out, const float* __restrict__ bias,
+                      const __nv_bfloat16* __restrict__ addend, const __nv_bfloat16* __restrict__ mask, int relu, int nx,
+                      int ny, int nz, WalkGeo g, int* err, int withhold, unsigned long long lim) {
+    constexpr int NCOL = COUT < 32 ? 32 : COUT;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;  // weights | ring | barriers
+    unsigned char* basep = smem_raw + (base - raw);
+    const uint32_t ring = base + g.wbytes;
+    const uint32_t bar_full = ring + g.stages * g.slot;
+    const uint32_t bar_empty = bar_full + 8 * kStagesWalk;
+    const uint32_t bar_w = bar_empty + 8 * kStagesWalk;
+    const uint32_t bar_accf = bar_w + 8, bar_acce = bar_accf + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(basep + (bar_acce + 16 - base));
+    volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);  // the first output plane without a sum
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int chunk = blockIdx.x / g.tiles, p0 = (blockIdx.x - chunk * g.tiles) * 128;
+    const int z0 = chunk * g.zc, nout = min(g.zc, nz - z0), nk = nout + 2;
+    const int x0 = p0 / g.pitch, off0 = p0 - x0 * g.pitch;
+    // a withheld step is numbered by taps, as in conv3_fwd_kernel
+    withhold = blockIdx.x != 0 || withhold < 0 ? -1 : min(withhold / 9, nk - 1);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < g.stages; ++s) {
+            mbar_init(bar_full + 8 * s, 128);  // the producer threads
+            mbar_init(bar_empty + 8 * s, 1);
+        }
+        mbar_init(bar_w, 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(bar_accf + 8 * b, 1);
+            mbar_init(bar_acce + 8 * b, 4);
+        }
+        mbar_init_fence();
+        *s_fail = 1 << 30;
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_slot), 2 * NCOL);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0 && lane == 0) {
+        mbar_expect_tx(bar_w, (uint32_t)(27 * COUT * (cin0 + (nparts > 1 ? cin1 : 0)) * 2));
+        for (int part = 0; part < nparts; ++part)
+            for (int j = 0; j < 9; ++j) {
+                const uint32_t at = part ? base + g.w1 + j * 3 * COUT * cin1 * 2 : base + j * 3 * COUT * cin0 * 2;
+                tma_load_2d(at, part ? &wm1 : &wm0, bar_w, 0, 3 * j * COUT);
+            }
+    } else if (warp >= 6) {
+        // input planes: step k is issued when its slot is free and handed over lag steps later, so that the
+        // copies of up to lag + 1 steps are in flight (a product of plane o waits for three steps: lag + 3
+        // <= stages)
+        const int tid = threadIdx.x - 192, lag = min(2, g.stages - 3);
+        auto hand_over = [&](int k) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (k != withhold) mbar_arrive(bar_full + 8 * (k % g.stages));
+        };
+        int k = 0;
+        for (; k < nk; ++k) {
+            const int s = k % g.stages;
+            if (k >= g.stages && !mbar_wait(bar_empty + 8 * s, ((k / g.stages) & 1) ^ 1, err, lim)) break;
+            const int zz = z0 + k - 1;
+            const bool zin = zz >= 0 && zz < nz;
+            uint32_t a = ring + s * g.slot;
+            for (int part = 0; part < nparts; ++part) {
+                const int cin = part ? cin1 : cin0, lg = cin == 16 ? 1 : cin == 32 ? 2 : 3;  // log2 of its 8-channel parts
+                const __nv_bfloat16* src = (part ? xin1 : xin0) + (long)zz * nx * ny * cin;
+                for (int e = tid; e < (g.rows * g.pitch) << lg; e += 128) {
+                    const int pos = e >> lg, c = e & ((1 << lg) - 1);
+                    const int r = (int)__umulhi((unsigned)pos, g.mpitch), yy = pos - r * g.pitch - 1, xx = x0 - 1 + r;
+                    const bool in = zin && xx >= 0 && xx < nx && yy >= 0 && yy < ny;
+                    cp_async16_zfill(a + c * g.lbo + 16 * pos, in ? src + ((long)xx * ny + yy) * cin + 8 * c : xin0, in ? 16 : 0);
+                }
+                a += cin / 8 * g.lbo;
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (lag == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+            else asm volatile("cp.async.wait_group 1;" ::: "memory");
+            if (k >= lag) hand_over(k - lag);
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");  // none in flight when the CTA exits
+        for (int j = max(k - lag, 0); j < k; ++j) hand_over(j);
+    } else if (warp == 1 && lane == 0) {
+        constexpr uint32_t idesc = idesc_bf16_f32(128, COUT, 0, 0);
+        int have = 0, o = 0;
+        bool ok = mbar_wait(bar_w, 0, err, lim);
+        for (; ok && o < nout; ++o) {
+            const uint32_t acc = tmem + (o & 1) * NCOL;
+            if (o >= 2) ok = mbar_wait(bar_acce + 8 * (o & 1), ((o >> 1) & 1) ^ 1, err, lim);
+            for (int dz = 0; ok && dz < 3; ++dz) {
+                const int k = o + dz, s = k % g.stages;
+                if (k >= have) {
+                    ok = mbar_wait(bar_full + 8 * s, (k / g.stages) & 1, err, lim);
+                    if (!ok) break;
+                    have = k + 1;
+                }
+                tc_fence_after();
+                uint32_t a = ring + s * g.slot + 16 * off0;
+                for (int part = 0; part < nparts; ++part) {
+                    const int cin = part ? cin1 : cin0;
+                    const uint32_t b = base + (part ? g.w1 : 0) + dz * 9 * COUT * cin * 2;
+                    if (cin == 16) walk_taps<COUT, 16>(acc, a, b, g, idesc, (dz | part) == 0);
+                    else if (cin == 32) walk_taps<COUT, 32>(acc, a, b, g, idesc, (dz | part) == 0);
+                    else walk_taps<COUT, 64>(acc, a, b, g, idesc, (dz | part) == 0);
+                    a += cin / 8 * g.lbo;
+                }
+            }
+            if (!ok) break;
+            umma_commit(bar_empty + 8 * (o % g.stages));  // input plane o has had its last use
+            umma_commit(bar_accf + 8 * (o & 1));
+        }
+        if (o < nout) {
+            *s_fail = o;
+            __threadfence_block();
+            umma_commit(bar_accf + 8 * (o & 1));  // tracks the MMAs already issued
+        }
+    } else if (warp >= 2 && warp < 6) {
+        const int q = warp & 3;
+        const int p = p0 + q * 32 + lane;
+        const int x = p / g.pitch, y = p - x * g.pitch;
+        for (int o = 0; o < nout; ++o) {
+            const bool ready = mbar_wait(bar_accf + 8 * (o & 1), (o >> 1) & 1, err);
+            if (!__all_sync(0xffffffffu, ready && *s_fail > o)) break;
+            tc_fence_after();
+            float acc[COUT];
+#pragma unroll
+            for (int c = 0; c < COUT; c += 16) tmem_ld16(tmem + (o & 1) * NCOL + ((uint32_t)(q * 32) << 16) + c, acc + c);
+            tmem_wait_ld();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_acce + 8 * (o & 1));
+            if (x < nx && y < ny)
+                store_voxel<COUT>(acc, ((long)(z0 + o) * nx + x) * ny + y, out, bias, addend, mask, relu);
+        }
+    }
+    if (warp == 0 && lane == 0) mbar_wait(bar_w, 0, err);  // no copy in flight when the CTA exits
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem, 2 * NCOL);
     }
 }
 
@@ -342,13 +555,13 @@ bool map_volume(CUtensorMap* m, const void* p, int c, int nx, int ny, int nz, in
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// [27 * cout][cin] weights, box (cin, cout)
-bool map_weights(CUtensorMap* m, const void* p, int cin, int cout) {
+// [27 * cout][cin] weights, box (cin, taps * cout)
+bool map_weights(CUtensorMap* m, const void* p, int cin, int cout, int taps = 1) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cin, (cuuint64_t)27 * cout};
     const cuuint64_t strides[1] = {(cuuint64_t)cin * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)cin, (cuuint32_t)cout};
+    const cuuint32_t box[2] = {(cuuint32_t)cin, (cuuint32_t)(taps * cout)};
     const cuuint32_t es[2] = {1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, es,
               CU_TENSOR_MAP_INTERLEAVE_NONE, swz(cin * 2), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -364,6 +577,39 @@ TileGeo tile_geo(int nx, int ny) {
     g.xt = 128 / g.yt;
     g.nty = (ny + g.yt - 1) / g.yt;
     g.ntx = (nx + g.xt - 1) / g.xt;
+    return g;
+}
+
+// The walk kernel's geometry for a layer, or stages = 0 where the weights and four input planes do not fit
+// shared memory (64 channels on both sides, 96 into 32: those stay with conv3_fwd_kernel).
+WalkGeo walk_geo(int nx, int ny, int nz, int cin0, int cin1, int cout) {
+    WalkGeo g{};
+    g.pitch = ny + 2;
+    if (g.pitch > 4096) return g;
+    g.mpitch = (unsigned)((0x100000000ull + g.pitch - 1) / g.pitch);
+    g.tiles = (nx * g.pitch + 127) / 128;
+    // a tile starts up to ny + 1 positions into its first row and reads two rows and two positions further
+    g.rows = 2 + (128 + ny + 1 + g.pitch - 1) / g.pitch;
+    g.lbo = (g.rows * g.pitch * 16 + 127) / 128 * 128;
+    // (the last rows of a tile's last taps may lie past the block: 64 bytes of slack)
+    g.slot = ((cin0 + cin1) / 8 * g.lbo + 64 + 1023) / 1024 * 1024;
+    // (a part's weights start on a 1024-byte boundary, the period of the widest swizzle)
+    g.w1 = (27 * cout * cin0 * 2 + 1023) / 1024 * 1024;
+    g.wbytes = g.w1 + (27 * cout * cin1 * 2 + 1023) / 1024 * 1024;
+    // CTAs per SM: what the registers hold (56, 88 and 152 a thread for 16, 32 and 64 outputs), where the weights and a
+    // ring of four planes fit their share of the shared memory
+    int ctas = cout == 16 ? 3 : cout == 32 ? 2 : 1;
+    for (; ctas >= 1; --ctas) {
+        const int room = (226 * 1024 / ctas - 2560 - g.wbytes) / g.slot;
+        if (226 * 1024 / ctas - 2560 > g.wbytes && room >= 4) {
+            g.stages = std::min(room, kStagesWalk);
+            break;
+        }
+    }
+    if (!g.stages) return g;
+    // one wave of CTAs
+    const long slots = (long)ctas * wp_sm_count();
+    g.zc = (int)(((long)g.tiles * nz + slots - 1) / slots);
     return g;
 }
 
@@ -392,6 +638,24 @@ cudaError_t launch_fwd(const CUtensorMap& x0, const CUtensorMap& w0, const CUten
     const long tiles = (long)tg.nty * tg.ntx * nz;
     k<<<(unsigned)tiles, kThreads, smem, s>>>(x0, w0, x1, w1, cin0, cin1, nparts, out, bias, addend, mask, relu, nx, ny,
                                               nz, tg, err, wh, lim);
+    return cudaGetLastError();
+}
+
+template <int COUT>
+cudaError_t launch_walk(const __nv_bfloat16* x0, const CUtensorMap& w0, const __nv_bfloat16* x1, const CUtensorMap& w1,
+                        int cin0, int cin1, int nparts, __nv_bfloat16* out, const float* bias,
+                        const __nv_bfloat16* addend, const __nv_bfloat16* mask, int relu, int nx, int ny, int nz,
+                        WalkGeo g, int* err, cudaStream_t s) {
+    const size_t smem = 1024 + (size_t)g.wbytes + (size_t)g.stages * g.slot + 16 * kStagesWalk + 8 + 32 + 32;
+    int wh = -1;
+    unsigned long long lim = wptc::kWaitLimitNs;
+    if (!wp_take_withhold(WP_WAIT_SITE_CONV_PIPELINE, s, &wh, &lim)) wh = -1;
+    auto k = conv3_walk_kernel<COUT>;
+    cudaError_t e = wp_set_smem(k, smem);
+    if (e != cudaSuccess) return e;
+    const unsigned ctas = (unsigned)(g.tiles * ((nz + g.zc - 1) / g.zc));
+    k<<<ctas, kWalkThreads, smem, s>>>(x0, w0, x1, w1, cin0, cin1, nparts, out, bias, addend, mask, relu, nx, ny, nz, g,
+                                       err, wh, lim);
     return cudaGetLastError();
 }
 
@@ -444,13 +708,20 @@ wp_status wp_conv3_forward_impl(void* out, const void* x0, int cin0, const void*
         return WP_ERR_INVALID_ARG;
     }
     const TileGeo tg = tile_geo(nx, ny);
+    const WalkGeo wg = walk_geo(nx, ny, nz, cin0, x1 ? cin1 : 0, cout);
+    // (its copies need 16-byte aligned inputs, as the tensor maps do)
+    const bool walk = wg.stages > 0 && (((uintptr_t)x0 | (uintptr_t)x1) & 15u) == 0;
+    auto maps = [&](CUtensorMap* mx, CUtensorMap* mw, const void* x, const void* w, int cin) {
+        return walk ? map_weights(mw, w, cin, cout, 3)
+                    : map_volume(mx, x, cin, nx, ny, nz, tg.yt, tg.xt) && map_weights(mw, w, cin, cout);
+    };
     CUtensorMap mx0, mw0, mx1, mw1;
-    if (!map_volume(&mx0, x0, cin0, nx, ny, nz, tg.yt, tg.xt) || !map_weights(&mw0, w0, cin0, cout)) {
+    if (!maps(&mx0, &mw0, x0, w0, cin0)) {
         wp_set_error_msg("wp_conv3_forward: tensor map encoding failed");
         return WP_ERR_CUDA;
     }
     if (x1) {
-        if (!map_volume(&mx1, x1, cin1, nx, ny, nz, tg.yt, tg.xt) || !map_weights(&mw1, w1, cin1, cout)) {
+        if (!maps(&mx1, &mw1, x1, w1, cin1)) {
             wp_set_error_msg("wp_conv3_forward: tensor map encoding failed");
             return WP_ERR_CUDA;
         }
@@ -466,10 +737,15 @@ wp_status wp_conv3_forward_impl(void* out, const void* x0, int cin0, const void*
     auto mk = static_cast<const __nv_bfloat16*>(mask);
     cudaError_t e;
     const int tok = wp_prof_start(s);
+    auto go = [&](auto fwd, auto walkk) {
+        return walk ? walkk(static_cast<const __nv_bfloat16*>(x0), mw0, static_cast<const __nv_bfloat16*>(x1), mw1, cin0, cin1,
+                            nparts, o, bias, ad, mk, relu, nx, ny, nz, wg, err, s)
+                    : fwd(mx0, mw0, mx1, mw1, cin0, cin1, nparts, o, bias, ad, mk, relu, nx, ny, nz, tg, err, s);
+    };
     switch (cout) {
-        case 16: e = launch_fwd<16>(mx0, mw0, mx1, mw1, cin0, cin1, nparts, o, bias, ad, mk, relu, nx, ny, nz, tg, err, s); break;
-        case 32: e = launch_fwd<32>(mx0, mw0, mx1, mw1, cin0, cin1, nparts, o, bias, ad, mk, relu, nx, ny, nz, tg, err, s); break;
-        default: e = launch_fwd<64>(mx0, mw0, mx1, mw1, cin0, cin1, nparts, o, bias, ad, mk, relu, nx, ny, nz, tg, err, s); break;
+        case 16: e = go(launch_fwd<16>, launch_walk<16>); break;
+        case 32: e = go(launch_fwd<32>, launch_walk<32>); break;
+        default: e = go(launch_fwd<64>, launch_walk<64>); break;
     }
     const double flops = 2.0 * 27.0 * (cin0 + (x1 ? cin1 : 0)) * cout * (double)nx * ny * nz;
     wp_prof_stop(tok, "conv3_tc", flops, s);
