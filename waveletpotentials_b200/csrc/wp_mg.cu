@@ -32,6 +32,7 @@ namespace {
 
 constexpr double kEps = 1e-12;
 constexpr int kMaxLevels = 24;
+constexpr unsigned char kUniLean = 3;  // Lvl::uni
 
 template <typename T>
 struct Lvl {
@@ -40,8 +41,9 @@ struct Lvl {
     const float* ay;
     const float* az;
     const float* fyc; // y-face fractions in cell layout: fyc[cell] = ay of the cell's lower y face
-    const unsigned char* uni; // per (x, z) row, at [z nx + x]: 1 when every face fraction the row's
-                              // stencils read (interior faces only) is exactly 1
+    const unsigned char* uni; // per (x, z) row, at [z nx + x]: nonzero when every face fraction the row's
+                              // stencils read (interior faces only) is exactly 1; kUniLean when moreover
+                              // all its x and z neighbours exist and its z factors are plane nz / 2's
     const T* glo[3];  // per-axis factor of the lower face, 0 at the wall
     const T* ghi[3];  // per-axis factor of the upper face, 0 at the wall
     const double* d[3];
@@ -86,17 +88,38 @@ __global__ void __launch_bounds__(256) jacobi_kernel(T* __restrict__ dst, const 
     dst[i] = dg > (T)kEps ? ((T)1 - w) * c + w * (f[i] - od) / dg : (T)0;
 }
 
-// Column walker: the row of cell (x, y, z) for z = z0, z0+1, ... with the z neighbours and the
-// z-face fraction carried in registers, so each v and az value of the column is loaded once;
-// in-plane neighbours come through L1 (they are loaded by the neighbouring threads of the CTA).
-template <typename T, typename TV, bool PROL>
+// diagonal of cell (x, y, z)
+template <typename T>
+__device__ __forceinline__ T cell_diag(const Lvl<T>& L, int x, int y, int z) {
+    const int nx = L.nx, ny = L.ny;
+    const long i = y + (long)x * ny + (long)z * nx * ny;
+    const long iax = y + (long)x * ny + (long)z * (nx + 1) * ny, iay = y + (long)x * (ny + 1) + (long)z * nx * (ny + 1);
+    T d = 0;
+    if (y > 0) d += (T)L.ay[iay] * L.glo[1][y];
+    if (y < ny - 1) d += (T)L.ay[iay + 1] * L.ghi[1][y];
+    if (x > 0) d += (T)L.ax[iax] * L.glo[0][x];
+    if (x < nx - 1) d += (T)L.ax[iax + ny] * L.ghi[0][x];
+    if (z > 0) d += (T)L.az[i] * L.glo[2][z];
+    if (z < L.nz - 1) d += (T)L.az[i + (long)nx * ny] * L.ghi[2][z];
+    return d;
+}
+
+// Column walker for any extents: the cell (x, y, z) for z = z0, z0+1, ... with the z neighbours and the
+// z-face fraction carried in registers, so each v and az value of the column is loaded once; in-plane
+// neighbours come through L1 (they are loaded by the neighbouring threads of the CTA).  A step gives the
+// residual, w / diagonal and the centre value as QCol's does (t = -c, rd = 1 where inactive with RD, t = 0
+// without), and rows flagged kUniLean read no fractions and divide by nothing.  201 x 150 x 101: a finest sweep 29.8 -> 21
+// us, the restriction 37 -> 22.5, the FP64 defect 55 -> 36 (1.9 TB/s of L2 and DRAM traffic, latency of the column).
+template <typename T, typename TV, bool PROL, bool RD = true>
 struct ZCol {
     const Lvl<T>& L;
     const TV* __restrict__ v;
     const TV* __restrict__ vc;
     int ncx, ncy, x, y, z;
-    long sxy, i, iax, iay, sax, say;
-    T vm, vcur, az_lo, gxl, gxh, gyl, gyh;
+    long sxy, i;
+    bool lean;        // the diagonal of a lean row is above kEps
+    unsigned char un; // row flag of plane z
+    T vm, vcur, az_lo, w, gxl, gxh, gyl, gyh, gzl, gzh, dgu, rdu;
 
     __device__ __forceinline__ T V(long ii, int xx, int yy, int zz) const {
         T r = (T)v[ii];
@@ -105,66 +128,117 @@ struct ZCol {
     }
 
     __device__ __forceinline__ ZCol(const Lvl<T>& L_, const TV* v_, const TV* vc_, int ncx_, int ncy_, int x_, int y_,
-                                    int z0)
-        : L(L_), v(v_), vc(vc_), ncx(ncx_), ncy(ncy_), x(x_), y(y_), z(z0) {
+                                    int z0, T w_ = (T)1)
+        : L(L_), v(v_), vc(vc_), ncx(ncx_), ncy(ncy_), x(x_), y(y_), z(z0), w(w_) {
         sxy = (long)L.nx * L.ny;
         i = y + (long)x * L.ny + z0 * sxy;
-        sax = (long)(L.nx + 1) * L.ny;
-        say = (long)L.nx * (L.ny + 1);
-        iax = y + (long)x * L.ny + z0 * sax;
-        iay = y + (long)x * (L.ny + 1) + z0 * say;
         vm = z0 > 0 ? V(i - sxy, x, y, z0 - 1) : (T)0;
         vcur = V(i, x, y, z0);
+        un = L.uni[(long)z0 * L.nx + x];
         az_lo = z0 > 0 ? (T)L.az[i] : (T)0;
         gxl = L.glo[0][x];
         gxh = L.ghi[0][x];
         gyl = L.glo[1][y];
         gyh = L.ghi[1][y];
+        gzl = L.glo[2][L.nz >> 1];
+        gzh = L.ghi[2][L.nz >> 1];
+        dgu = gyl + gyh + gxl + gxh + gzl + gzh;
+        lean = dgu > (T)kEps;
+        rdu = RD ? w / dgu : (T)1;
     }
 
-    // diag, off-diagonal sum and centre value of the current cell; then advances one plane
-    __device__ __forceinline__ void step(T& dg, T& od, T& c) {
+    // the current cell; then advances one plane
+    __device__ __forceinline__ void step(T f, T& t, T& rd, T& c) {
         const int nx = L.nx, ny = L.ny, nz = L.nz;
-        T d = 0, o = 0, cf;
-        if (y > 0) { cf = (T)L.ay[iay] * gyl; d += cf; o -= cf * V(i - 1, x, y - 1, z); }
-        if (y < ny - 1) { cf = (T)L.ay[iay + 1] * gyh; d += cf; o -= cf * V(i + 1, x, y + 1, z); }
-        if (x > 0) { cf = (T)L.ax[iax] * gxl; d += cf; o -= cf * V(i - ny, x - 1, y, z); }
-        if (x < nx - 1) { cf = (T)L.ax[iax + ny] * gxh; d += cf; o -= cf * V(i + ny, x + 1, y, z); }
-        T vp = 0, az_hi = 0;
-        if (z > 0) { cf = az_lo * L.glo[2][z]; d += cf; o -= cf * vm; }
-        if (z < nz - 1) {
-            vp = V(i + sxy, x, y, z + 1);
-            az_hi = (T)L.az[i + sxy];
-            cf = az_hi * L.ghi[2][z];
-            d += cf;
-            o -= cf * vp;
-        }
-        dg = d;
-        od = o;
+        const unsigned char u = un;
+        const bool zp = z < nz - 1;
+        un = zp ? L.uni[(long)(z + 1) * nx + x] : 0;
+        const T vp = zp ? V(i + sxy, x, y, z + 1) : (T)0;
+        const T ym = y > 0 ? V(i - 1, x, y - 1, z) : (T)0, yp = y < ny - 1 ? V(i + 1, x, y + 1, z) : (T)0;
+        const T xm = x > 0 ? V(i - ny, x - 1, y, z) : (T)0, xp = x < nx - 1 ? V(i + ny, x + 1, y, z) : (T)0;
         c = vcur;
+        if (u == kUniLean && lean) {
+            // a wall's y factor is 0
+            T s = fma(gyl, ym, f);
+            s = fma(gyh, yp, s);
+            s = fma(gxl, xm, s);
+            s = fma(gxh, xp, s);
+            s = fma(gzl, vm, s);
+            s = fma(gzh, vp, s);
+            t = fma(-dgu, c, s);
+            rd = rdu;
+            az_lo = (T)1;
+        } else {
+            T fyl = 1, fyh = 1, fxl = 1, fxh = 1, az_hi = 1;
+            if (!u) {
+                const long iax = y + (long)x * ny + (long)z * (nx + 1) * ny, iay = y + (long)x * (ny + 1) + (long)z * nx * (ny + 1);
+                fyl = (T)L.ay[iay];
+                fyh = (T)L.ay[iay + 1];
+                fxl = (T)L.ax[iax];
+                fxh = (T)L.ax[iax + ny];
+                if (zp) az_hi = (T)L.az[i + sxy];
+            }
+            T d = 0, o = 0, cf;
+            if (y > 0) { cf = fyl * gyl; d += cf; o -= cf * ym; }
+            if (y < ny - 1) { cf = fyh * gyh; d += cf; o -= cf * yp; }
+            if (x > 0) { cf = fxl * gxl; d += cf; o -= cf * xm; }
+            if (x < nx - 1) { cf = fxh * gxh; d += cf; o -= cf * xp; }
+            if (z > 0) { cf = az_lo * L.glo[2][z]; d += cf; o -= cf * vm; }
+            if (zp) { cf = az_hi * L.ghi[2][z]; d += cf; o -= cf * vp; }
+            const bool act = d > (T)kEps;
+            t = act ? (f - o) - d * c : RD ? -c : (T)0;
+            rd = act && RD ? w / d : (T)1;
+            az_lo = az_hi;
+        }
         vm = vcur;
         vcur = vp;
-        az_lo = az_hi;
         i += sxy;
-        iax += sax;
-        iay += say;
         ++z;
     }
 };
 
+// p64 given: the swept values are added to it instead of stored (jacobi_q_body's ACC form)
 template <typename T, bool PROL>
 __global__ void __launch_bounds__(256) jacobi_z_kernel(T* __restrict__ dst, const T* __restrict__ src,
                                                        const T* __restrict__ f, Lvl<T> L, T w,
-                                                       const T* __restrict__ vc, int ncx, int ncy, int zc) {
+                                                       const T* __restrict__ vc, int ncx, int ncy, int zc,
+                                                       double* __restrict__ p64 = nullptr) {
+    wp_pdl_enter();
     const int y = blockIdx.x * 32 + threadIdx.x, x = blockIdx.y * 8 + threadIdx.y;
     const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, L.nz);
     if (y >= L.ny || x >= L.nx || z0 >= z1) return;
-    ZCol<T, T, PROL> col(L, src, vc, ncx, ncy, x, y, z0);
+    ZCol<T, T, PROL> col(L, src, vc, ncx, ncy, x, y, z0, w);
     for (int z = z0; z < z1; ++z) {
         const long i = col.i;
-        T dg, od, c;
-        col.step(dg, od, c);
-        dst[i] = dg > (T)kEps ? ((T)1 - w) * c + w * (f[i] - od) / dg : (T)0;
+        T t, rd, c;
+        col.step(f[i], t, rd, c);
+        const T o = fma(rd, t, c);
+        if (p64) p64[i] += (double)o;
+        else dst[i] = o;
+    }
+}
+
+// the first sweep from v = 0 (jacobi0_q_body) for any extents
+template <typename T>
+__global__ void __launch_bounds__(256) jacobi0_z_kernel(T* __restrict__ dst, const T* __restrict__ f, Lvl<T> L, T w,
+                                                        int zc) {
+    wp_pdl_enter();
+    const int y = blockIdx.x * 32 + threadIdx.x, x = blockIdx.y * 8 + threadIdx.y;
+    const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, L.nz);
+    if (y >= L.ny || x >= L.nx || z0 >= z1) return;
+    const T du = L.glo[1][y] + L.ghi[1][y] + L.glo[0][x] + L.ghi[0][x] + L.glo[2][L.nz >> 1] + L.ghi[2][L.nz >> 1];
+    const T rdu = w / du;
+    long i = y + (long)x * L.ny + (long)z0 * L.nx * L.ny;
+    for (int z = z0; z < z1; ++z, i += (long)L.nx * L.ny) {
+        const T fv = f[i];
+        T o;
+        if (L.uni[(long)z * L.nx + x] == kUniLean && du > (T)kEps) {
+            o = rdu * fv;
+        } else {
+            const T d = cell_diag(L, x, y, z);
+            o = d > (T)kEps ? w * fv / d : (T)0;
+        }
+        dst[i] = o;
     }
 }
 
@@ -1178,9 +1252,11 @@ __global__ void fyc_kernel(float* __restrict__ fyc, const float* __restrict__ ay
 // uni[z nx + x] = 1 when every face of row (x, z) that a stencil reads is exactly 1: the lower y
 // faces of y >= 1 (fyc), the x faces x and x + 1 and the z faces z and z + 1 that are interior.  One
 // warp per row.
+// kUniLean when moreover every x and z neighbour exists and the z factors are those of plane nz / 2
+// (glo, ghi: the FP64 tables, whose FP32 rounding then agrees too).  A 2D level has no z faces.
 __global__ void uniform_rows_kernel(unsigned char* __restrict__ uni, const float* __restrict__ ax,
                                     const float* __restrict__ fyc, const float* __restrict__ az, int nx, int ny,
-                                    int nz) {
+                                    int nz, const double* __restrict__ glo, const double* __restrict__ ghi) {
     const long rows = (long)nx * nz;
     const int lane = threadIdx.x & 31;
     for (long r = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5; r < rows; r += ((long)gridDim.x * blockDim.x) >> 5) {
@@ -1197,7 +1273,9 @@ __global__ void uniform_rows_kernel(unsigned char* __restrict__ uni, const float
             if (z < nz - 1) ok = ok && az[i + sxy + y] == 1.f;
         }
         ok = __all_sync(0xffffffffu, ok);
-        if (lane == 0) uni[r] = ok ? 1 : 0;
+        const bool lean = x > 0 && x < nx - 1 && (nz == 1 || (z > 0 && z < nz - 1)) && glo[z] == glo[nz >> 1] &&
+                          ghi[z] == ghi[nz >> 1];
+        if (lane == 0) uni[r] = ok ? (lean ? kUniLean : 1) : 0;
     }
 }
 
@@ -1208,6 +1286,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) resid_restrict_z_kernel(T* __restrict__ fc, const T* __restrict__ v,
                                                                const T* __restrict__ f, Lvl<T> L, int ncx, int ncy,
                                                                int ncz, int czc) {
+    wp_pdl_enter();
     __shared__ T red[8][16];
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int y = blockIdx.x * 32 + tx, x = blockIdx.y * 8 + ty;
@@ -1220,19 +1299,20 @@ __global__ void __launch_bounds__(256) resid_restrict_z_kernel(T* __restrict__ f
         const double sx = L.d[0][x0] + (x0 + 1 < L.nx ? L.d[0][x0 + 1] : 0.0);
         wxy = (T)(L.d[1][y] / sy * (L.d[0][x] / sx));
     }
-    ZCol<T, T, false> col(L, v, nullptr, 0, 0, in ? x : 0, in ? y : 0, 2 * cz0);
+    ZCol<T, T, false, false> col(L, v, nullptr, 0, 0, in ? x : 0, in ? y : 0, 2 * cz0);
     for (int cz = cz0; cz < cz1; ++cz) {
         T acc = 0;
         const int zb = 2 * cz;
-        const double sz = L.d[2][zb] + (zb + 1 < L.nz ? L.d[2][zb + 1] : 0.0);
+        double sz = 0.0;
+        if constexpr (sizeof(T) == 8) sz = L.d[2][zb] + (zb + 1 < L.nz ? L.d[2][zb + 1] : 0.0);
         for (int k = 0; k < 2; ++k) {
             const int z = zb + k;
             if (z < L.nz && in) {
-                const long i = col.i;
-                T dg, od, c;
-                col.step(dg, od, c);
-                const T r = dg > (T)kEps ? f[i] - (dg * c + od) : (T)0;
-                acc += (T)(L.d[2][z] / sz) * wxy * r;
+                // FP32: the same FP64 quotient, rounded once, from the level's table
+                const T wz = sizeof(T) == 4 ? (T)L.rwz[z] : (T)(L.d[2][z] / sz);
+                T t, one, c;
+                col.step(f[col.i], t, one, c);
+                acc += wz * wxy * t;
             }
         }
         acc += __shfl_xor_sync(0xffffffffu, acc, 1);
@@ -2027,17 +2107,17 @@ __global__ void __launch_bounds__(256) defect64_z_kernel(float* __restrict__ r32
                                                          const float* __restrict__ f, Lvl<double> L, double m,
                                                          const double* __restrict__ msum, double* __restrict__ acc,
                                                          int zc) {
+    wp_pdl_enter();
     const int y = blockIdx.x * 32 + threadIdx.x, x = blockIdx.y * 8 + threadIdx.y;
     const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, L.nz);
     if (msum) m = msum[0] / fmax(msum[1], 1.0);  // mean of f over the active cells, computed on the device
     double s2 = 0.0;
     if (y < L.ny && x < L.nx && z0 < z1) {
-        ZCol<double, TP, false> col(L, p, nullptr, 0, 0, x, y, z0);
+        ZCol<double, TP, false, false> col(L, p, nullptr, 0, 0, x, y, z0);
         for (int z = z0; z < z1; ++z) {
             const long i = col.i;
-            double dg, od, c;
-            col.step(dg, od, c);
-            const double r = dg > kEps ? ((double)f[i] - m) - (dg * c + od) : 0.0;
+            double r, one, c;
+            col.step((double)f[i] - m, r, one, c);
             if (r32) r32[i] = (float)r;
             s2 += r * r;
         }
@@ -2532,8 +2612,8 @@ void launch_jacobi(const Level& L, T* dst, const T* src, const T* f, T w, int zc
         else if (var == 2) wp_launch_pdl(jacobi_q_mb_kernel<T, 4>, g, 256, 0, s, dst, src, f, V, w, zc, nullptr);
         else wp_launch_pdl(jacobi_q_kernel<T>, g, 256, 0, s, dst, src, f, V, w, zc, nullptr);
     } else {
-        jacobi_z_kernel<T, false><<<grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s>>>(dst, src, f, V, w, nullptr,
-                                                                                          0, 0, zc);
+        wp_launch_pdl(jacobi_z_kernel<T, false>, grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, dst, src, f, V, w,
+                      (const T*)nullptr, 0, 0, zc, (double*)nullptr);
     }
 }
 
@@ -2541,12 +2621,18 @@ void launch_jacobi(const Level& L, T* dst, const T* src, const T* f, T w, int zc
 // One FP32 sweep of src whose result is added to p64 instead of stored (the level's tuned one-sweep
 // quad kernel); false when the level's kernel has no such form (the caller then stores and adds).
 bool jacobi_acc_ok(const Level& L, const void* src, const void* f, const double* p64) {
-    return quad_ok(L) && al16(src) && al16(f) && al16(p64) && (L.var[kZcJacobi] <= 2 || L.var[kZcJacobi] == 5);
+    if (!quad_ok(L)) return true;
+    return al16(src) && al16(f) && al16(p64) && (L.var[kZcJacobi] <= 2 || L.var[kZcJacobi] == 5);
 }
 void launch_jacobi_acc(const Level& L, const float* src, const float* f, float w, int zc, double* p64,
                        cudaStream_t s) {
     const int var = L.var[kZcJacobi];
     const Lvl<float> V = view<float>(L);
+    if (!quad_ok(L)) {
+        wp_launch_pdl(jacobi_z_kernel<float, false>, grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, (float*)nullptr,
+                      src, f, V, w, (const float*)nullptr, 0, 0, zc, p64);
+        return;
+    }
     const dim3 g(wp_cdiv((size_t)L.n[0] * (L.n[1] / 4), 256), wp_cdiv(L.n[2], zc));
     if (var == 1) wp_launch_pdl(jacobi_q_mb_kernel<float, 3, true>, g, 256, 0, s, nullptr, src, f, V, w, zc, p64);
     else if (var == 5) {
@@ -2586,7 +2672,7 @@ void launch_resid_restrict(const Level& L, const Level& C, T* fc, const T* v, co
         else wp_launch_pdl(resid_restrict_q_kernel<T>, g, 256, 0, s, fc, v, f, V, C.n[0], C.n[1], C.n[2], czc);
     } else {
         const dim3 g(wp_cdiv(L.n[1], 32), wp_cdiv(L.n[0], 8), wp_cdiv(C.n[2], czc));
-        resid_restrict_z_kernel<T><<<g, dim3(32, 8), 0, s>>>(fc, v, f, V, C.n[0], C.n[1], C.n[2], czc);
+        wp_launch_pdl(resid_restrict_z_kernel<T>, g, dim3(32, 8), 0, s, fc, v, f, V, C.n[0], C.n[1], C.n[2], czc);
     }
 }
 
@@ -2607,8 +2693,8 @@ void launch_defect64(const Level& L, float* r32, const TP* p, const float* f, do
         }
         wp_launch_pdl(defect64_q_kernel<TP>, g, 256, 0, s, r32, p, f, V, m, msum, acc, zc);
     } else {
-        defect64_z_kernel<TP><<<grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s>>>(r32, p, f, V, m, msum, acc,
-                                                                                       zc);
+        wp_launch_pdl(defect64_z_kernel<TP>, grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, r32, p, f, V, m, msum,
+                      acc, zc);
     }
 }
 
@@ -2618,8 +2704,8 @@ void launch_prolong_tri(const Level& L, const Level& C, T* v, const T* vc, cudaS
         const dim3 g(wp_cdiv((size_t)L.n[0] * (L.n[1] / 4), 256), L.n[2]);
         wp_launch_pdl(prolong_tri_q_kernel<T>, g, 256, 0, s, v, vc, L.n[0], L.n[1], L.n[2], C.n[0], C.n[1], C.n[2]);
     } else {
-        prolong_tri_add_kernel<T><<<grid_of(L.n[0], L.n[1], L.n[2]), dim3(32, 8), 0, s>>>(v, vc, L.n[0], L.n[1], L.n[2],
-                                                                                         C.n[0], C.n[1], C.n[2]);
+        wp_launch_pdl(prolong_tri_add_kernel<T>, grid_of(L.n[0], L.n[1], L.n[2]), dim3(32, 8), 0, s, v, vc, L.n[0], L.n[1],
+                      L.n[2], C.n[0], C.n[1], C.n[2]);
     }
 }
 
@@ -2759,17 +2845,6 @@ wp_status build_hierarchy(wp_mgfrac3d* h, const float* ax, const float* ay, cons
         WP_KERNEL("fyc", 8.0 * L.cells, s,
                   fyc_kernel<<<std::min<unsigned>(wp_cdiv(L.cells, 256), 4096), 256, 0, s>>>(L.fyc, L.frac[1], n[0],
                                                                                              n[1], L.cells));
-        WP_CUDA_TRY(cudaMalloc((void**)&L.uni, (size_t)n[0] * n[2]));
-        WP_KERNEL("uniform_rows", 16.0 * L.cells, s,
-                  uniform_rows_kernel<<<std::min<unsigned>(wp_cdiv((long)n[0] * n[2] * 32, 256), 4096), 256, 0, s>>>(
-                      L.uni, L.frac[0], L.fyc, L.frac[2], n[0], n[1], n[2]));
-        {
-            std::vector<unsigned char> u((size_t)n[0] * n[2]);
-            WP_CUDA_TRY(cudaMemcpyAsync(u.data(), L.uni, u.size(), cudaMemcpyDeviceToHost, s));
-            WP_CUDA_TRY(cudaStreamSynchronize(s));
-            L.uni_rows = 0;
-            for (unsigned char b : u) L.uni_rows += b != 0;
-        }
         if (dims == 3 && fz_level_ok(n)) {
             const int ntiles = (n[0] / fz::TX) * (n[1] / fz::TY);
             WP_CUDA_TRY(cudaMalloc((void**)&L.tuni, (size_t)ntiles * n[2]));
@@ -2828,6 +2903,17 @@ wp_status build_hierarchy(wp_mgfrac3d* h, const float* ax, const float* ay, cons
         WP_CUDA_TRY(cudaMalloc((void**)&L.tab32, sizeof(float) * t32.size()));
         WP_CUDA_TRY(cudaMemcpy(L.tab64, t64.data(), sizeof(double) * t64.size(), cudaMemcpyHostToDevice));
         WP_CUDA_TRY(cudaMemcpy(L.tab32, t32.data(), sizeof(float) * t32.size(), cudaMemcpyHostToDevice));
+        WP_CUDA_TRY(cudaMalloc((void**)&L.uni, (size_t)n[0] * n[2]));
+        WP_KERNEL("uniform_rows", 16.0 * L.cells, s,
+                  uniform_rows_kernel<<<std::min<unsigned>(wp_cdiv((long)n[0] * n[2] * 32, 256), 4096), 256, 0, s>>>(
+                      L.uni, L.frac[0], L.fyc, L.frac[2], n[0], n[1], n[2], view<double>(L).glo[2], view<double>(L).ghi[2]));
+        {
+            std::vector<unsigned char> u((size_t)n[0] * n[2]);
+            WP_CUDA_TRY(cudaMemcpyAsync(u.data(), L.uni, u.size(), cudaMemcpyDeviceToHost, s));
+            WP_CUDA_TRY(cudaStreamSynchronize(s));
+            L.uni_rows = 0;
+            for (unsigned char b : u) L.uni_rows += b != 0;
+        }
         WP_CUDA_TRY(cudaMalloc((void**)&L.v, sizeof(float) * L.cells));
         WP_CUDA_TRY(cudaMalloc((void**)&L.t, sizeof(float) * L.cells));
         WP_CUDA_TRY(cudaMalloc((void**)&L.f, sizeof(float) * L.cells));
@@ -3231,6 +3317,13 @@ wp_status vcycle(wp_mgfrac3d* h, int l, const T* f, int nu1, int nu2, T w, int p
                 const dim3 gq(wp_cdiv((size_t)L.n[0] * (L.n[1] / 4), 256), wp_cdiv(L.n[2], zc));
                 WP_KERNEL(l == 0 ? "jacobi0_finest" : "jacobi0", (double)L.cells * 2.0 * sizeof(T) + frac_bytes(L), s,
                           wp_launch_pdl(jacobi0_q_kernel<T>, gq, 256, 0, s, Bufs<T>::t(L), f, view<T>(L), w, zc));
+                std::swap(Bufs<T>::v(L), Bufs<T>::t(L));
+                pre = nu1 - 1;
+            } else if (nu1 > 0 && !quad_ok(L)) {
+                const int zc = level_zc(L, kZcJacobi);
+                WP_KERNEL(l == 0 ? "jacobi0_finest" : "jacobi0", (double)L.cells * 2.0 * sizeof(T) + frac_bytes(L), s,
+                          wp_launch_pdl(jacobi0_z_kernel<T>, grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s,
+                                        Bufs<T>::t(L), f, view<T>(L), w, zc));
                 std::swap(Bufs<T>::v(L), Bufs<T>::t(L));
                 pre = nu1 - 1;
             } else {
