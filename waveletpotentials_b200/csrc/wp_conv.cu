@@ -5,7 +5,8 @@
 // Layouts.  Activations: [z][x][y][c] BF16 (c fastest), c in {16, 32, 64}.  Weights of one input
 // part: [tap][cout][cin] BF16 with tap = (dz * 3 + dx) * 3 + dy, offsets d - 1 (zero padding).
 //
-// Forward / input-gradient kernel (implicit GEMM, K-major operands).  A CTA owns a tile of
+// Forward / input-gradient kernels (implicit GEMM, K-major operands).  Layers whose weights and a ring of input
+// planes fit shared memory take conv3_walk_kernel (described there), the others conv3_fwd_kernel: a CTA owns a tile of
 // M = 128 voxels of one z plane (yt consecutive y times xt consecutive x, yt * xt = 128) and all
 // cout outputs.  K runs over (input part, tap, cin): per tap a TMA load brings the shifted
 // [128 voxels][cin] block of the input (out-of-range voxels arrive as zeros = the padding) and the

@@ -6,7 +6,8 @@
 // :600-631; CDF4.6: :925-942, :983-1002, reflection :336-375, :716-752; base matrices :773-874).
 // Output layout (Mallat order): [base (4+ext) | d level 2 (4) | d level 3 (8) | ... | d level L-1 (n/2)].
 //
-// B200 design: one CTA owns a tile of C whole lines (C = 32/16/8/4 columns) staged in shared
+// B200 design.  CDF3.7 and CDF4.6 lines of up to 512 samples take dwt_line_kernel (in place, described there).
+// The others, dwt_tile_kernel: one CTA owns a tile of C whole lines (C = 32/16/8/4 columns) staged in shared
 // memory as S[position][column] (column pitch C+1 so both the y-contiguous load and the
 // column-parallel lifting are bank-conflict free).  All levels run on chip; global memory is
 // read once and written once per pass, coalesced along y for every axis (for the x and z axes
