@@ -233,8 +233,11 @@ CUWHHD_API wp_status wp_mgfrac3d_iterate64_view(wp_mgfrac3d* h, const double** o
 CUWHHD_API wp_status wp_mgfrac3d_destroy(wp_mgfrac3d* h);
 /* Tile-shape autotuner (no reference counterpart): times the column-walking stencil kernels of
    every level (Jacobi sweep, fused residual-restriction, FP64 defect) over candidate z-chunks and
-   keeps the fastest per level; results are independent of the choice.  Synchronous; overwrites
-   the handle's work arrays (not the FP64 iterate).  Choices are cached per device and extents for
+   keeps the fastest per level; results are independent of these choices.  It also times level 0's
+   V(2,2) cycle as two fused kernels, and the levels below it as one persistent launch (kinds 4 and 3
+   of wp_mgfrac3d_set_tile): those agree with the kernel-by-kernel cycle to FP32 rounding, so pin
+   them where every bit has to repeat from process to process.  Synchronous; overwrites the handle's
+   work arrays (not the FP64 iterate).  Choices are cached per device and extents for
    the process.  Each candidate is timed as the median of single launches, after an L2 flush for
    levels larger than 16 MB, among chunks that give at least two CTAs per SM (when the level has
    that many columns).  wp_mgfrac3d_tiles reports 3 chunks per level (jacobi, restrict, defect),

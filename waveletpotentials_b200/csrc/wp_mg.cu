@@ -107,10 +107,12 @@ __device__ __forceinline__ T cell_diag(const Lvl<T>& L, int x, int y, int z) {
 // Column walker for any extents: the cell (x, y, z) for z = z0, z0+1, ... with the z neighbours and the
 // z-face fraction carried in registers, so each v and az value of the column is loaded once; in-plane
 // neighbours come through L1 (they are loaded by the neighbouring threads of the CTA).  A step gives the
-// residual, w / diagonal and the centre value as QCol's does (t = -c, rd = 1 where inactive with RD, t = 0
-// without), and rows flagged kUniLean read no fractions and divide by nothing.  201 x 150 x 101: a finest sweep 29.8 -> 21
+// swept value (SWEEP) or the residual, 0 where the cell is inactive.
+// LEAN: rows flagged kUniLean read no fractions and divide by nothing.  201 x 150 x 101: a finest sweep 29.8 -> 21
 // us, the restriction 37 -> 22.5, the FP64 defect 55 -> 36 (1.9 TB/s of L2 and DRAM traffic, latency of the column).
-template <typename T, typename TV, bool PROL, bool RD = true>
+// Without it the operations are QCol's: where a level of whole quads could run either kernel (by the tuner's choice or
+// an argument's alignment), its one-cell kernel takes that form, so that the choice never shows in the bits.
+template <typename T, typename TV, bool PROL, bool SWEEP, bool LEAN>
 struct ZCol {
     const Lvl<T>& L;
     const TV* __restrict__ v;
@@ -143,12 +145,12 @@ struct ZCol {
         gzl = L.glo[2][L.nz >> 1];
         gzh = L.ghi[2][L.nz >> 1];
         dgu = gyl + gyh + gxl + gxh + gzl + gzh;
-        lean = dgu > (T)kEps;
-        rdu = RD ? w / dgu : (T)1;
+        lean = LEAN && dgu > (T)kEps;
+        rdu = SWEEP && LEAN ? w / dgu : (T)1;
     }
 
-    // the current cell; then advances one plane
-    __device__ __forceinline__ void step(T f, T& t, T& rd, T& c) {
+    // the current cell, f its right-hand side; then advances one plane
+    __device__ __forceinline__ T step(T f) {
         const int nx = L.nx, ny = L.ny, nz = L.nz;
         const unsigned char u = un;
         const bool zp = z < nz - 1;
@@ -156,7 +158,8 @@ struct ZCol {
         const T vp = zp ? V(i + sxy, x, y, z + 1) : (T)0;
         const T ym = y > 0 ? V(i - 1, x, y - 1, z) : (T)0, yp = y < ny - 1 ? V(i + 1, x, y + 1, z) : (T)0;
         const T xm = x > 0 ? V(i - ny, x - 1, y, z) : (T)0, xp = x < nx - 1 ? V(i + ny, x + 1, y, z) : (T)0;
-        c = vcur;
+        const T c = vcur;
+        T r;
         if (u == kUniLean && lean) {
             // a wall's y factor is 0
             T s = fma(gyl, ym, f);
@@ -165,8 +168,8 @@ struct ZCol {
             s = fma(gxh, xp, s);
             s = fma(gzl, vm, s);
             s = fma(gzh, vp, s);
-            t = fma(-dgu, c, s);
-            rd = rdu;
+            const T t = fma(-dgu, c, s);
+            r = SWEEP ? fma(rdu, t, c) : t;
             az_lo = (T)1;
         } else {
             T fyl = 1, fyh = 1, fxl = 1, fxh = 1, az_hi = 1;
@@ -185,20 +188,25 @@ struct ZCol {
             if (x < nx - 1) { cf = fxh * gxh; d += cf; o -= cf * xp; }
             if (z > 0) { cf = az_lo * L.glo[2][z]; d += cf; o -= cf * vm; }
             if (zp) { cf = az_hi * L.ghi[2][z]; d += cf; o -= cf * vp; }
-            const bool act = d > (T)kEps;
-            t = act ? (f - o) - d * c : RD ? -c : (T)0;
-            rd = act && RD ? w / d : (T)1;
+            if (LEAN) {
+                const T t = (f - o) - d * c;
+                r = SWEEP ? fma(w / d, t, c) : t;
+            } else {
+                r = SWEEP ? ((T)1 - w) * c + w * (f - o) / d : f - (d * c + o);
+            }
+            if (!(d > (T)kEps)) r = (T)0;
             az_lo = az_hi;
         }
         vm = vcur;
         vcur = vp;
         i += sxy;
         ++z;
+        return r;
     }
 };
 
 // p64 given: the swept values are added to it instead of stored (jacobi_q_body's ACC form)
-template <typename T, bool PROL>
+template <typename T, bool PROL, bool LEAN>
 __global__ void __launch_bounds__(256) jacobi_z_kernel(T* __restrict__ dst, const T* __restrict__ src,
                                                        const T* __restrict__ f, Lvl<T> L, T w,
                                                        const T* __restrict__ vc, int ncx, int ncy, int zc,
@@ -207,12 +215,10 @@ __global__ void __launch_bounds__(256) jacobi_z_kernel(T* __restrict__ dst, cons
     const int y = blockIdx.x * 32 + threadIdx.x, x = blockIdx.y * 8 + threadIdx.y;
     const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, L.nz);
     if (y >= L.ny || x >= L.nx || z0 >= z1) return;
-    ZCol<T, T, PROL> col(L, src, vc, ncx, ncy, x, y, z0, w);
+    ZCol<T, T, PROL, true, LEAN> col(L, src, vc, ncx, ncy, x, y, z0, w);
     for (int z = z0; z < z1; ++z) {
         const long i = col.i;
-        T t, rd, c;
-        col.step(f[i], t, rd, c);
-        const T o = fma(rd, t, c);
+        const T o = col.step(f[i]);
         if (p64) p64[i] += (double)o;
         else dst[i] = o;
     }
@@ -451,7 +457,10 @@ __device__ __forceinline__ void jacobi_q_body(T* __restrict__ dst, const T* __re
 
 // The first sweep from v = 0: every neighbour and the centre are 0, so the sweep is
 // (1 - w) 0 + w (f - 0) / diag, which reads only f and (outside uniform rows) the fractions for the
-// diagonal -- the same value as jacobi_q_body on a zeroed v, with no v to clear or read.
+// diagonal -- the same value as jacobi_q_body on a zeroed v (whose diagonal sums rounded products: mul_rn keeps
+// them from being fused into the sum), with no v to clear or read.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 template <typename T, bool CG = false>
 __device__ __forceinline__ void jacobi0_q_body(T* __restrict__ dst, const T* __restrict__ f, const Lvl<T>& L, T w,
                                                int zc, int bx, int by, int tid) {
@@ -499,12 +508,12 @@ __device__ __forceinline__ void jacobi0_q_body(T* __restrict__ dst, const T* __r
         for (int k = 0; k < 4; ++k) {
             const int y = y0 + k;
             T d = 0;
-            if (y > 0) d += (T)fyl.a[k] * gyl[k];
-            if (y < ny - 1) d += (T)(k < 3 ? fyl.a[k + 1] : fyu) * gyh[k];
-            if (xm) d += (T)fxl.a[k] * gxl;
-            if (xp) d += (T)fxu.a[k] * gxh;
-            if (z > 0) d += azl.a[k] * gzl;
-            if (zp) d += azu.a[k] * gzh;
+            if (y > 0) d += mul_rn((T)fyl.a[k], gyl[k]);
+            if (y < ny - 1) d += mul_rn((T)(k < 3 ? fyl.a[k + 1] : fyu), gyh[k]);
+            if (xm) d += mul_rn((T)fxl.a[k], gxl);
+            if (xp) d += mul_rn((T)fxu.a[k], gxh);
+            if (z > 0) d += mul_rn(azl.a[k], gzl);
+            if (zp) d += mul_rn(azu.a[k], gzh);
             out.a[k] = d > (T)kEps ? ((T)1 - w) * (T)0 + w * (fv.a[k] - (T)0) / d : (T)0;
         }
         st4(dst + i, out);
@@ -1325,7 +1334,7 @@ __global__ void uniform_rows_kernel(unsigned char* __restrict__ uni, const float
 // Fused residual + restriction: each thread walks one fine column, the 2 x 2 children in (y, x)
 // are combined with a lane shuffle and a shared-memory exchange, the 2 children in z in registers.
 // Coarse value = sum of (dx_x dx_y dx_z / sums) weighted fine residuals (cuRestrict3D.cu:801-970).
-template <typename T>
+template <typename T, bool LEAN>
 __global__ void __launch_bounds__(256) resid_restrict_z_kernel(T* __restrict__ fc, const T* __restrict__ v,
                                                                const T* __restrict__ f, Lvl<T> L, int ncx, int ncy,
                                                                int ncz, int czc) {
@@ -1342,7 +1351,7 @@ __global__ void __launch_bounds__(256) resid_restrict_z_kernel(T* __restrict__ f
         const double sx = L.d[0][x0] + (x0 + 1 < L.nx ? L.d[0][x0 + 1] : 0.0);
         wxy = (T)(L.d[1][y] / sy * (L.d[0][x] / sx));
     }
-    ZCol<T, T, false, false> col(L, v, nullptr, 0, 0, in ? x : 0, in ? y : 0, 2 * cz0);
+    ZCol<T, T, false, false, LEAN> col(L, v, nullptr, 0, 0, in ? x : 0, in ? y : 0, 2 * cz0);
     for (int cz = cz0; cz < cz1; ++cz) {
         T acc = 0;
         const int zb = 2 * cz;
@@ -1353,9 +1362,7 @@ __global__ void __launch_bounds__(256) resid_restrict_z_kernel(T* __restrict__ f
             if (z < L.nz && in) {
                 // FP32: the same FP64 quotient, rounded once, from the level's table
                 const T wz = sizeof(T) == 4 ? (T)L.rwz[z] : (T)(L.d[2][z] / sz);
-                T t, one, c;
-                col.step(f[col.i], t, one, c);
-                acc += wz * wxy * t;
+                acc += wz * wxy * col.step(f[col.i]);
             }
         }
         acc += __shfl_xor_sync(0xffffffffu, acc, 1);
@@ -2169,7 +2176,7 @@ __global__ void __launch_bounds__(256) defect64_kernel(float* __restrict__ r32, 
 // walls the operator's null space is the constant on the active cells, so a right-hand side stored
 // in FP32 carries an incompatible constant part of FP32 rounding size that floors the residual
 // (about 2e-10 relative at 64^3); the tolerance-driven solve removes that mean in FP64.
-template <typename TP>
+template <typename TP, bool LEAN>
 __global__ void __launch_bounds__(256) defect64_z_kernel(float* __restrict__ r32, const TP* __restrict__ p,
                                                          const float* __restrict__ f, Lvl<double> L, double m,
                                                          const double* __restrict__ msum, double* __restrict__ acc,
@@ -2180,11 +2187,10 @@ __global__ void __launch_bounds__(256) defect64_z_kernel(float* __restrict__ r32
     if (msum) m = msum[0] / fmax(msum[1], 1.0);  // mean of f over the active cells, computed on the device
     double s2 = 0.0;
     if (y < L.ny && x < L.nx && z0 < z1) {
-        ZCol<double, TP, false, false> col(L, p, nullptr, 0, 0, x, y, z0);
+        ZCol<double, TP, false, false, LEAN> col(L, p, nullptr, 0, 0, x, y, z0);
         for (int z = z0; z < z1; ++z) {
             const long i = col.i;
-            double r, one, c;
-            col.step((double)f[i] - m, r, one, c);
+            const double r = col.step((double)f[i] - m);
             if (r32) r32[i] = (float)r;
             s2 += r * r;
         }
@@ -2679,8 +2685,9 @@ void launch_jacobi(const Level& L, T* dst, const T* src, const T* f, T w, int zc
         else if (var == 2) wp_launch_pdl(jacobi_q_mb_kernel<T, 4>, g, 256, 0, s, dst, src, f, V, w, zc, nullptr);
         else wp_launch_pdl(jacobi_q_kernel<T>, g, 256, 0, s, dst, src, f, V, w, zc, nullptr);
     } else {
-        wp_launch_pdl(jacobi_z_kernel<T, false>, grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, dst, src, f, V, w,
-                      (const T*)nullptr, 0, 0, zc, (double*)nullptr);
+        wp_launch_pdl(quad_ok(L) ? jacobi_z_kernel<T, false, false> : jacobi_z_kernel<T, false, true>,
+                      grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, dst, src, f, V, w, (const T*)nullptr, 0, 0, zc,
+                      (double*)nullptr);
     }
 }
 
@@ -2696,7 +2703,7 @@ void launch_jacobi_acc(const Level& L, const float* src, const float* f, float w
     const int var = L.var[kZcJacobi];
     const Lvl<float> V = view<float>(L);
     if (!quad_ok(L)) {
-        wp_launch_pdl(jacobi_z_kernel<float, false>, grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, (float*)nullptr,
+        wp_launch_pdl(jacobi_z_kernel<float, false, true>, grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, (float*)nullptr,
                       src, f, V, w, (const float*)nullptr, 0, 0, zc, p64);
         return;
     }
@@ -2739,7 +2746,8 @@ void launch_resid_restrict(const Level& L, const Level& C, T* fc, const T* v, co
         else wp_launch_pdl(resid_restrict_q_kernel<T>, g, 256, 0, s, fc, v, f, V, C.n[0], C.n[1], C.n[2], czc);
     } else {
         const dim3 g(wp_cdiv(L.n[1], 32), wp_cdiv(L.n[0], 8), wp_cdiv(C.n[2], czc));
-        wp_launch_pdl(resid_restrict_z_kernel<T>, g, dim3(32, 8), 0, s, fc, v, f, V, C.n[0], C.n[1], C.n[2], czc);
+        wp_launch_pdl(quad_ok(L) ? resid_restrict_z_kernel<T, false> : resid_restrict_z_kernel<T, true>, g, dim3(32, 8), 0, s,
+                      fc, v, f, V, C.n[0], C.n[1], C.n[2], czc);
     }
 }
 
@@ -2760,8 +2768,8 @@ void launch_defect64(const Level& L, float* r32, const TP* p, const float* f, do
         }
         wp_launch_pdl(defect64_q_kernel<TP>, g, 256, 0, s, r32, p, f, V, m, msum, acc, zc);
     } else {
-        wp_launch_pdl(defect64_z_kernel<TP>, grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, r32, p, f, V, m, msum,
-                      acc, zc);
+        wp_launch_pdl(quad_ok(L) ? defect64_z_kernel<TP, false> : defect64_z_kernel<TP, true>,
+                      grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, r32, p, f, V, m, msum, acc, zc);
     }
 }
 
@@ -3418,7 +3426,7 @@ wp_status vcycle(wp_mgfrac3d* h, int l, const T* f, int nu1, int nu2, T w, int p
             // first post-sweep reads v + P vc directly (prolongation fused into the sweep)
             const int zc = level_zc(L, kZcJacobi);
             WP_KERNEL("jacobi_prolong", (double)L.cells * (3.0 * sizeof(T) + 12.0) + (double)C.cells * sizeof(T), s,
-                      jacobi_z_kernel<T, true><<<grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s>>>(
+                      jacobi_z_kernel<T, true, true><<<grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s>>>(
                           Bufs<T>::t(L), Bufs<T>::v(L), f, view<T>(L), w, Bufs<T>::v(C), C.n[0], C.n[1], zc));
             T* tmp = Bufs<T>::v(L);
             Bufs<T>::v(L) = Bufs<T>::t(L);
@@ -5090,8 +5098,8 @@ extern "C" CUWHHD_API wp_status wp_mgfrac2d_destroy(wp_mgfrac2d* h) {
 // ---- internal hooks used by the batched path (wp_batch.cu)
 // ------------------------------------------------------------------ tile-shape autotuner
 // Per level, times the column kernels (FP32 Jacobi sweep, fused residual-restriction, FP64 defect)
-// over candidate z-chunks with CUDA events and keeps the fastest.  Results do not depend on the
-// chunk (each cell's arithmetic is the same; only the grid shape changes).  Timings are cached per
+// over variants and candidate z-chunks with CUDA events and keeps the fastest.  Results do not depend
+// on either (each cell's arithmetic is the same).  Timings are cached per
 // (device, kernel, extents) for the process, so later handles of the same shapes skip the search.
 namespace {
 
