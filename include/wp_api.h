@@ -233,10 +233,10 @@ CUWHHD_API wp_status wp_mgfrac3d_iterate64_view(wp_mgfrac3d* h, const double** o
 CUWHHD_API wp_status wp_mgfrac3d_destroy(wp_mgfrac3d* h);
 /* Tile-shape autotuner (no reference counterpart): times the column-walking stencil kernels of
    every level (Jacobi sweep, fused residual-restriction, FP64 defect) over candidate z-chunks and
-   keeps the fastest per level; results are independent of these choices.  It also times level 0's
-   V(2,2) cycle as two fused kernels, and the levels below it as one persistent launch (kinds 4 and 3
-   of wp_mgfrac3d_set_tile): those agree with the kernel-by-kernel cycle to FP32 rounding, so pin
-   them where every bit has to repeat from process to process.  Synchronous; overwrites the handle's
+   keeps the fastest per level; results are independent of these choices.  It also times the
+   levels below the finest as one persistent launch (the same bits) and level 0's V(2,2) cycle as two
+   fused kernels, which agree with the kernel-by-kernel cycle to FP32 rounding (kinds 3 and 4 of
+   wp_mgfrac3d_set_tile; pin kind 4 where every bit has to repeat from process to process).  Synchronous; overwrites the handle's
    work arrays (not the FP64 iterate).  Choices are cached per device and extents for
    the process.  Each candidate is timed as the median of single launches, after an L2 flush for
    levels larger than 16 MB, among chunks that give at least two CTAs per SM (when the level has
@@ -506,14 +506,14 @@ CUWHHD_API wp_status wp_batch_results(wp_batch* h, double* max_abs_div, double* 
    branch of the graph (a while-node per grid).  WP_BATCH_PERSISTENT: every grid's solve runs in ONE
    persistent kernel inside the graph (one 1024-thread CTA per SM) that takes (grid, level, pass)
    tiles from a device work queue: per grid a program of the phases of one refinement step (first
-   sweep from zero, sweeps, residual restriction, the single-CTA coarse cycle, prolongation, the
+   sweep from zero, sweeps, residual restriction, the coarse cycle of one CTA, prolongation, the
    sweep that adds to the FP64 iterate, FP64 defect and stopping rule) repeated until the rule stops
    it, the grids advancing independently; the divergence, gradient update, max|div u| and recovery
    of the grids run on the graph's branches before and after it.  Same per-cell arithmetic, same
    results as WP_BATCH_GRAPH (up to the order of the FP64 norm reductions).  tile_cells: cells per
    work-queue tile (0 = 32768).  Needs trilinear V(nu1, nu2) cycles with nu1, nu2 >= 1 from a zero
    start and, per grid, levels whose y extent is a multiple of 4 down to a coarse level of at most
-   4096 cells whose pack fits the CTA's shared memory; WP_ERR_UNSUPPORTED otherwise (the mode stays
+   4096 cells; WP_ERR_UNSUPPORTED otherwise (the mode stays
    as it was).  Every wait of the persistent kernel is bounded (WP_ERR_DEVICE_WAIT from
    wp_batch_results when one gave up). */
 #define WP_BATCH_GRAPH 0

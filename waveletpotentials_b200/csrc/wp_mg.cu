@@ -1176,6 +1176,13 @@ __global__ void __launch_bounds__(256, 2) defect64_qp_kernel(float* __restrict__
     }
 }
 
+// 3/4 of the parent and 1/4 of its neighbour, rounded once (the quarter is exact).  Spelled out: every prolongation
+// gives the same bits.
+template <typename T>
+__device__ __forceinline__ T tri_mix(T parent, T neighbour) {
+    return fma((T)0.75, parent, (T)0.25 * neighbour);
+}
+
 // trilinear prolongation (prolong_tri_add_kernel) on quads: one 128-bit read-modify-write of v
 template <typename T, bool CG = false>
 __device__ __forceinline__ void prolong_tri_q_body(T* __restrict__ v, const T* __restrict__ vc, int nx, int ny, int nz,
@@ -1189,7 +1196,6 @@ __device__ __forceinline__ void prolong_tri_q_body(T* __restrict__ v, const T* _
     if (qx < 0 || qx >= ncx) qx = px;
     if (qz < 0 || qz >= ncz) qz = pz;
     const long sc = (long)ncx * ncy;
-    const T a = (T)0.75, b = (T)0.25;
     const long i = y0 + (long)x * ny + (long)z * nx * ny;
     Q4<T> out = ldq<CG>(v + i);
     // the quad's coarse y values along one coarse (x, z) row: cy0 - 1, cy0, cy0 + 1, cy0 + 2, with the
@@ -1221,7 +1227,7 @@ __device__ __forceinline__ void prolong_tri_q_body(T* __restrict__ v, const T* _
             T P0, Q0, P1, Q1;
             PQ(r0, k, P0, Q0);
             PQ(r1, k, P1, Q1);
-            out.a[k] += a * (a * P0 + b * Q0) + b * (a * P1 + b * Q1);
+            out.a[k] += tri_mix(tri_mix(P0, Q0), tri_mix(P1, Q1));
         }
     } else {
         const Row4 r00 = row4(px, pz), r10 = row4(qx, pz), r01 = row4(px, qz), r11 = row4(qx, qz);
@@ -1232,9 +1238,8 @@ __device__ __forceinline__ void prolong_tri_q_body(T* __restrict__ v, const T* _
             PQ(r10, k, P10, Q10);
             PQ(r01, k, P01, Q01);
             PQ(r11, k, P11, Q11);
-            const T lo = a * (a * P00 + b * Q00) + b * (a * P10 + b * Q10);
-            const T hi = a * (a * P01 + b * Q01) + b * (a * P11 + b * Q11);
-            out.a[k] += a * lo + b * hi;
+            const T lo = tri_mix(tri_mix(P00, Q00), tri_mix(P10, Q10)), hi = tri_mix(tri_mix(P01, Q01), tri_mix(P11, Q11));
+            out.a[k] += tri_mix(lo, hi);
         }
     }
     st4(v + i, out);
@@ -1259,7 +1264,6 @@ __global__ void __launch_bounds__(256) prolong_tri_q_kernel(T* __restrict__ v, c
     if (qx < 0 || qx >= ncx) qx = px;
     const long sc = (long)ncx * ncy, sxy = (long)nx * ny, i = y0 + (long)x * ny + 2 * pz * sxy;
     const bool two = 2 * pz + 1 < nz;
-    const T a = (T)0.75, b = (T)0.25;
     Q4<T> o0 = ld4(v + i), o1 = o0;
     if (two) o1 = ld4(v + i + sxy);
     T pl[3][4];
@@ -1278,13 +1282,13 @@ __global__ void __launch_bounds__(256) prolong_tri_q_kernel(T* __restrict__ v, c
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int P = k < 2 ? 1 : 2, Q = k == 0 ? 0 : k == 1 ? 2 : k == 2 ? 1 : 3;
-            pl[j][k] = a * (a * r[0][P] + b * r[0][Q]) + b * (a * r[1][P] + b * r[1][Q]);
+            pl[j][k] = tri_mix(tri_mix(r[0][P], r[0][Q]), tri_mix(r[1][P], r[1][Q]));
         }
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        o0.a[k] += a * pl[1][k] + b * pl[0][k];
-        o1.a[k] += a * pl[1][k] + b * pl[2][k];
+        o0.a[k] += tri_mix(pl[1][k], pl[0][k]);
+        o1.a[k] += tri_mix(pl[1][k], pl[2][k]);
     }
     st4(v + i, o0);
     if (two) st4(v + i + sxy, o1);
@@ -1400,8 +1404,7 @@ __global__ void __launch_bounds__(256) prolong_tri_add_kernel(T* __restrict__ v,
     if (qx < 0 || qx >= ncx) qx = px;
     if (qy < 0 || qy >= ncy) qy = py;
     auto C = [&](int xx, int yy) -> T { return vc[yy + (long)xx * ncy]; };
-    const T a = (T)0.75, b = (T)0.25;
-    v[y + (long)x * ny] += a * (a * C(px, py) + b * C(px, qy)) + b * (a * C(qx, py) + b * C(qx, qy));
+    v[y + (long)x * ny] += tri_mix(tri_mix(C(px, py), C(px, qy)), tri_mix(C(qx, py), C(qx, qy)));
 }
 
 // prolong_tri_add_kernel for 3D levels of any extents, four fine planes per thread: the four coarse planes they read
@@ -1419,19 +1422,18 @@ __global__ void __launch_bounds__(256) prolong_tri_z_kernel(T* __restrict__ v, c
     if (qy < 0 || qy >= ncy) qy = py;
     const long sc = (long)ncx * ncy, sxy = (long)nx * ny, i = y + (long)x * ny + z0 * sxy;
     const long cpp = py + (long)px * ncy, cpq = qy + (long)px * ncy, cqp = py + (long)qx * ncy, cqq = qy + (long)qx * ncy;
-    const T a = (T)0.75, b = (T)0.25;
     T o[4], pl[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) o[k] = z0 + k < nz ? v[i + k * sxy] : (T)0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const T* c = vc + min(max(cz0 - 1 + j, 0), ncz - 1) * sc;  // (a missing plane repeats the parent's)
-        pl[j] = a * (a * c[cpp] + b * c[cpq]) + b * (a * c[cqp] + b * c[cqq]);
+        pl[j] = tri_mix(tri_mix(c[cpp], c[cpq]), tri_mix(c[cqp], c[cqq]));
     }
-    o[0] += a * pl[1] + b * pl[0];
-    o[1] += a * pl[1] + b * pl[2];
-    o[2] += a * pl[2] + b * pl[1];
-    o[3] += a * pl[2] + b * pl[3];
+    o[0] += tri_mix(pl[1], pl[0]);
+    o[1] += tri_mix(pl[1], pl[2]);
+    o[2] += tri_mix(pl[2], pl[1]);
+    o[3] += tri_mix(pl[2], pl[3]);
 #pragma unroll
     for (int k = 0; k < 4; ++k)
         if (z0 + k < nz) v[i + k * sxy] = o[k];
@@ -1651,346 +1653,6 @@ __global__ void __launch_bounds__(1024) coarse_cycle_kernel(CPack<T> P, int nu1,
     for (int i = threadIdx.x; i < n0; i += blockDim.x) out[i] = v[0][i];
 }
 
-// ---- FP32 coarse cycle on precomputed stencils ------------------------------------------------
-// The levels a coarse cycle can hold (cells <= kCoarseCells) keep their stencil per cell, SoA in
-// kCcf arrays of `cells` floats: [0..5] the face coefficients (fraction x spacing factor) in the order
-// row() applies them (y-, y+, x-, x+, z-, z+), 0 where row() skips the face; [6] row()'s diagonal
-// (their sum in that order); [7] the cell's restriction weight (T)(d_z / s_z) * (T)(d_y / s_y *
-// (d_x / s_x)) of resid_restrict.  A sweep then needs no index decomposition, no boundary branches
-// and no global loads: with v padded by one z plane on either side, the six neighbours are
-// i -+ 1, i -+ ny, i -+ nx ny, and a skipped face contributes 0 * (a finite neighbour).
-constexpr int kCcf = 8;
-constexpr size_t kLeanSmemMax = 226 * 1024;  // dynamic part; the level descriptors are static shared memory
-
-__global__ void cc_coeff_kernel(float* __restrict__ out, Lvl<float> L) {
-    const int nx = L.nx, ny = L.ny, nz = L.nz, cells = nx * ny * nz;
-    const long sxy = (long)nx * ny;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += gridDim.x * blockDim.x) {
-        const int y = i % ny, x = (i / ny) % nx, z = i / (nx * ny);
-        const long iax = y + (long)x * ny + (long)z * (nx + 1) * ny;
-        const long iay = y + (long)x * (ny + 1) + (long)z * nx * (ny + 1);
-        float c[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        float dg = 0.f;
-        if (y > 0) { c[0] = L.ay[iay] * L.glo[1][y]; dg += c[0]; }
-        if (y < ny - 1) { c[1] = L.ay[iay + 1] * L.ghi[1][y]; dg += c[1]; }
-        if (x > 0) { c[2] = L.ax[iax] * L.glo[0][x]; dg += c[2]; }
-        if (x < nx - 1) { c[3] = L.ax[iax + ny] * L.ghi[0][x]; dg += c[3]; }
-        if (z > 0) { c[4] = L.az[i] * L.glo[2][z]; dg += c[4]; }
-        if (z < nz - 1) { c[5] = L.az[i + sxy] * L.ghi[2][z]; dg += c[5]; }
-        const int x0 = x & ~1, y0 = y & ~1, zb = z & ~1;
-        const double sx = L.d[0][x0] + (x0 + 1 < nx ? L.d[0][x0 + 1] : 0.0);
-        const double sy = L.d[1][y0] + (y0 + 1 < ny ? L.d[1][y0 + 1] : 0.0);
-        const double sz = L.d[2][zb] + (zb + 1 < nz ? L.d[2][zb + 1] : 0.0);
-        const float wxy = (float)(L.d[1][y] / sy * (L.d[0][x] / sx));
-        const float wc = (float)(L.d[2][z] / sz) * wxy;
-        for (int k = 0; k < 6; ++k) out[(long)k * cells + i] = c[k];
-        out[6L * cells + i] = dg;
-        out[7L * cells + i] = wc;
-    }
-}
-
-struct LLev {
-    int nx, ny, nz;
-    const float* ccf; // kCcf x cells
-    float *v, *t;     // global v / t (written for the pack's finest level on exit)
-    const float* f;   // global right-hand side (read for the pack's finest level)
-};
-struct LPack {
-    LLev lv[kCoarseMax];
-    int n;
-};
-
-// shared floats a lean pack needs: per level v and t padded by a z plane on both sides, f, stencils
-// (cf_global: the stencils are read from global memory, not staged)
-inline long lean_smem_floats(const LPack& P, bool cf_global = false) {
-    long s = 0;
-    for (int l = 0; l < P.n; ++l) {
-        const long c = (long)P.lv[l].nx * P.lv[l].ny * P.lv[l].nz, p = (long)P.lv[l].nx * P.lv[l].ny;
-        s += 2 * (c + 2 * p) + c + (cf_global ? 0 : kCcf * c);
-    }
-    return s;
-}
-
-struct LS {
-    int nx, ny, nz, cells, nxy;
-    float *v, *t, *f; // v, t point past their lower padding plane
-    const float* cf;  // kCcf x cells
-};
-
-// off = -(sum of the present c_k * v_neighbour) in row()'s order; returns the centre value
-__device__ __forceinline__ float lean_off(const LS& S, const float* __restrict__ v, int i, float& od) {
-    const float* cf = S.cf;
-    const int n = S.cells;
-    float o = 0.f;
-    o -= cf[i] * v[i - 1];
-    o -= cf[n + i] * v[i + 1];
-    o -= cf[2 * n + i] * v[i - S.ny];
-    o -= cf[3 * n + i] * v[i + S.ny];
-    o -= cf[4 * n + i] * v[i - S.nxy];
-    o -= cf[5 * n + i] * v[i + S.nxy];
-    od = o;
-    return v[i];
-}
-
-__device__ __forceinline__ void lean_sweep(const LS& S, float* __restrict__ dst, const float* __restrict__ src, float w,
-                                           int i0, int step) {
-    for (int i = i0; i < S.cells; i += step) {
-        float od;
-        const float c = lean_off(S, src, i, od);
-        const float dg = S.cf[6 * S.cells + i];
-        dst[i] = dg > (float)kEps ? (1.f - w) * c + w * (S.f[i] - od) / dg : 0.f;
-    }
-}
-
-// (x, y, z) of cell i, and the step that adds `step` to i
-__device__ __forceinline__ void lean_coord(int i, int nx, int ny, int& x, int& y, int& z) {
-    y = i % ny;
-    x = (i / ny) % nx;
-    z = i / (nx * ny);
-}
-__device__ __forceinline__ void lean_advance(int& x, int& y, int& z, int bx, int by, int bz, int nx, int ny) {
-    y += by;
-    if (y >= ny) { y -= ny; ++x; }
-    x += bx;
-    if (x >= nx) { x -= nx; ++z; }
-    z += bz;
-}
-
-// residual of the fine level restricted to the coarse right-hand side (cc_restrict's sums and order):
-// first every fine cell's residual, by all threads, into the fine level's second buffer (free until
-// the post-sweeps write it), then each coarse cell's weighted sum of its children in the same order
-__device__ __forceinline__ void lean_restrict(const LS& F, const LS& C) {
-    const int B = blockDim.x;
-    const float* dgf = F.cf + 6L * F.cells;
-    for (int i = threadIdx.x; i < F.cells; i += B) {
-        float od;
-        const float c = lean_off(F, F.v, i, od);
-        const float dg = dgf[i];
-        F.t[i] = dg > (float)kEps ? F.f[i] - (dg * c + od) : 0.f;
-    }
-    __syncthreads();
-    int cx, cy, cz;
-    lean_coord(threadIdx.x, C.nx, C.ny, cx, cy, cz);
-    int bx, by, bz;
-    lean_coord(B, C.nx, C.ny, bx, by, bz);
-    const float* wcf = F.cf + 7L * F.cells;
-    for (int ci = threadIdx.x; ci < C.cells; ci += B) {
-        float tot[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-        for (int xo = 0; xo < 2; ++xo) {
-            const int x = 2 * cx + xo;
-            if (x >= F.nx) break;
-            for (int yo = 0; yo < 2; ++yo) {
-                const int y = 2 * cy + yo;
-                if (y >= F.ny) break;
-                float acc = 0.f;
-                for (int kz = 0; kz < 2; ++kz) {
-                    const int z = 2 * cz + kz;
-                    if (z >= F.nz) break;
-                    const int i = y + x * F.ny + z * F.nxy;
-                    acc += wcf[i] * F.t[i];
-                }
-                tot[xo][yo] = acc;
-            }
-        }
-        C.f[ci] = (tot[0][0] + tot[0][1]) + (tot[1][0] + tot[1][1]);
-        lean_advance(cx, cy, cz, bx, by, bz, C.nx, C.ny);
-    }
-}
-
-// v += P vc (cc_prolong's arithmetic)
-__device__ __forceinline__ void lean_prolong(const LS& F, const LS& C, int prolong) {
-    const int B = blockDim.x;
-    int x, y, z;
-    lean_coord(threadIdx.x, F.nx, F.ny, x, y, z);
-    int bx, by, bz;
-    lean_coord(B, F.nx, F.ny, bx, by, bz);
-    const int ncx = C.nx, ncy = C.ny, ncz = C.nz;
-    const float* vc = C.v;
-    for (int i = threadIdx.x; i < F.cells; i += B) {
-        const int px = x >> 1, py = y >> 1, pz = z >> 1;
-        if (prolong != WP_PROLONG_TRILINEAR) {
-            F.v[i] += vc[py + px * ncy + pz * C.nxy];
-        } else {
-            int qx = (x & 1) ? px + 1 : px - 1, qy = (y & 1) ? py + 1 : py - 1, qz = (z & 1) ? pz + 1 : pz - 1;
-            if (qx < 0 || qx >= ncx) qx = px;
-            if (qy < 0 || qy >= ncy) qy = py;
-            if (qz < 0 || qz >= ncz) qz = pz;
-            auto Cv = [&](int xx, int yy, int zz) -> float { return vc[yy + xx * ncy + zz * C.nxy]; };
-            const float a = 0.75f, b = 0.25f;
-            float acc;
-            if (ncz == 1 && F.nz == 1) {
-                acc = a * (a * Cv(px, py, 0) + b * Cv(px, qy, 0)) + b * (a * Cv(qx, py, 0) + b * Cv(qx, qy, 0));
-            } else {
-                const float lo =
-                    a * (a * Cv(px, py, pz) + b * Cv(px, qy, pz)) + b * (a * Cv(qx, py, pz) + b * Cv(qx, qy, pz));
-                const float hi =
-                    a * (a * Cv(px, py, qz) + b * Cv(px, qy, qz)) + b * (a * Cv(qx, py, qz) + b * Cv(qx, qy, qz));
-                acc = a * lo + b * hi;
-            }
-            F.v[i] += acc;
-        }
-        lean_advance(x, y, z, bx, by, bz, F.nx, F.ny);
-    }
-}
-
-// coarse_cycle_kernel<float> on the precomputed stencils, everything in shared memory: the same
-// cycle, the same arithmetic per cell, the same output buffer.  The pack's stencils are one
-// contiguous global block (the levels of at most kCoarseCells cells are allocated together, in
-// level order), copied with 128-bit loads that keep many requests in flight; the level
-// descriptors live in shared memory (no local-memory arrays), and thread 0 writes back the
-// ping-pong state of a level after its sweeps (every thread swaps its own copy in lockstep).
-// The body, run by one 1024-thread CTA (also as the coarse phase of mid_cycle_kernel, whose other
-// CTAs wrote the pack's right-hand side in the same grid: hence the L2 load of f).
-// CFG: the stencils stay in global memory (read through L1) and only v, t, f are staged, for a CTA
-// that keeps its shared memory small (the persistent batch kernel).
-template <bool CFG = false>
-__device__ __forceinline__ void lean_cycle(const LPack& P, int nu1, int nu2, float w, int citers, int prolong,
-                                           float* lean_smem) {
-    __shared__ LS S[kCoarseMax];
-    const int tid = threadIdx.x, B = blockDim.x;
-    long cf_floats = 0;
-    if (!CFG)
-        for (int l = 0; l < P.n; ++l) cf_floats += (long)kCcf * P.lv[l].nx * P.lv[l].ny * P.lv[l].nz;
-    if (tid == 0) {
-        long cfo = 0, off = cf_floats;
-        for (int l = 0; l < P.n; ++l) {
-            LS& q = S[l];
-            q.nx = P.lv[l].nx;
-            q.ny = P.lv[l].ny;
-            q.nz = P.lv[l].nz;
-            q.nxy = q.nx * q.ny;
-            q.cells = q.nxy * q.nz;
-            q.cf = CFG ? P.lv[l].ccf : lean_smem + cfo;
-            cfo += (long)kCcf * q.cells;
-            q.v = lean_smem + off + q.nxy;
-            off += q.cells + 2 * q.nxy;
-            q.t = lean_smem + off + q.nxy;
-            off += q.cells + 2 * q.nxy;
-            q.f = lean_smem + off;
-            off += q.cells;
-        }
-    }
-    if (!CFG) {
-        // stencils: 16-byte asynchronous copies (every level's block is a multiple of 16 bytes), all in
-        // flight at once while the buffers are cleared below, waited for before the first sweep
-        const char* g = reinterpret_cast<const char*>(P.lv[0].ccf);
-        char* d = reinterpret_cast<char*>(lean_smem);
-        const int n16 = (int)(cf_floats / 4);
-        for (int i = tid; i < n16; i += B) cp_async16(d + 16L * i, g + 16L * i);
-        cp_async_commit();
-    }
-    __syncthreads();
-    for (int l = 0; l < P.n; ++l) {
-        // padding planes stay zero; level 0 starts from v = 0 and the global f
-        const LS q = S[l];
-        for (int i = tid; i < q.cells + 2 * q.nxy; i += B) {
-            q.v[i - q.nxy] = 0.f;
-            q.t[i - q.nxy] = 0.f;
-        }
-        if (l == 0)
-            for (int i = tid; i < q.cells; i += B) q.f[i] = __ldcg(P.lv[0].f + i);
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-    for (int l = 0; l < P.n - 1; ++l) {
-        LS L = S[l];
-        if (l > 0) {
-            for (int i = tid; i < L.cells; i += B) L.v[i] = 0.f;
-            __syncthreads();
-        }
-        for (int k = 0; k < nu1; ++k) {
-            lean_sweep(L, L.t, L.v, w, tid, B);
-            __syncthreads();
-            float* tmp = L.v;
-            L.v = L.t;
-            L.t = tmp;
-        }
-        lean_restrict(L, S[l + 1]);
-        if (tid == 0) {
-            S[l].v = L.v;
-            S[l].t = L.t;
-        }
-        __syncthreads();
-    }
-    {
-        LS L = S[P.n - 1];
-        if (P.n > 1) {
-            for (int i = tid; i < L.cells; i += B) L.v[i] = 0.f;
-            __syncthreads();
-        }
-        if (L.cells <= 32) {
-            // a coarsest grid of at most 32 cells: one warp iterates alone, a cell per lane in
-            // registers, the neighbours' values by shuffle -- lean_sweep's arithmetic and order, the
-            // padding planes (indices outside the level) reading 0.  The result goes to the buffer the
-            // swaps of citers sweeps would leave it in.  A single cell has no interior face: its
-            // diagonal is 0 and the buffers already hold the 0 every sweep would write.
-            if (tid < 32 && L.cells > 1) {
-                const int n = L.cells, i = tid;
-                const bool own = i < n;
-                const int off[6] = {-1, 1, -L.ny, L.ny, -L.nxy, L.nxy};
-                float cfk[6], dg = 0.f, fv = 0.f, v = 0.f;
-#pragma unroll
-                for (int k = 0; k < 6; ++k) cfk[k] = own ? L.cf[k * n + i] : 0.f;
-                if (own) {
-                    dg = L.cf[6 * n + i];
-                    fv = L.f[i];
-                    v = L.v[i];
-                }
-                for (int it = 0; it < citers; ++it) {
-                    float o = 0.f;
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) {
-                        const int j = i + off[k];
-                        const float vj = __shfl_sync(0xffffffffu, v, j & 31);
-                        o -= cfk[k] * ((j >= 0 && j < n) ? vj : 0.f);
-                    }
-                    const float nv = dg > (float)kEps ? (1.f - w) * v + w * (fv - o) / dg : 0.f;
-                    v = own ? nv : v;
-                }
-                if (own) ((citers & 1) ? L.t : L.v)[i] = v;
-            }
-            if (citers & 1) {
-                float* tmp = L.v;
-                L.v = L.t;
-                L.t = tmp;
-            }
-        } else {
-            for (int k = 0; k < citers; ++k) {
-                lean_sweep(L, L.t, L.v, w, tid, B);
-                __syncthreads();
-                float* tmp = L.v;
-                L.v = L.t;
-                L.t = tmp;
-            }
-        }
-        if (tid == 0) {
-            S[P.n - 1].v = L.v;
-            S[P.n - 1].t = L.t;
-        }
-        __syncthreads();
-    }
-    for (int l = P.n - 2; l >= 0; --l) {
-        LS L = S[l];
-        lean_prolong(L, S[l + 1], prolong);
-        __syncthreads();
-        for (int k = 0; k < nu2; ++k) {
-            lean_sweep(L, L.t, L.v, w, tid, B);
-            __syncthreads();
-            float* tmp = L.v;
-            L.v = L.t;
-            L.t = tmp;
-        }
-        if (tid == 0) {
-            S[l].v = L.v;
-            S[l].t = L.t;
-        }
-        __syncthreads();
-    }
-    float* out = ((nu1 + nu2) & 1) ? P.lv[0].t : P.lv[0].v;
-    const float* v0 = S[0].v;
-    for (int i = tid; i < S[0].cells; i += B) out[i] = v0[i];
-}
-
 #include "wp_mg_cluster.cuh"
 
 // ---- persistent cycle below the finest level --------------------------------------------------
@@ -1998,10 +1660,11 @@ __device__ __forceinline__ void lean_cycle(const LPack& P, int nu1, int nu2, flo
 // as separate launches each sweep costs a launch, a ramp and a tail.  mid_cycle_kernel runs the whole
 // cycle below the finest level in one cooperative launch (one 1024-thread CTA per SM, all resident):
 // a list of phases -- first sweep from zero, sweeps, residual restriction, trilinear prolongation
-// and the single-CTA coarse cycle -- separated by grid barriers.  A phase runs the quad kernels'
-// bodies (the same arithmetic per cell) on virtual 256-thread blocks, four per CTA, with every load
-// of data written earlier in the grid taken through L2 (CG).  The host mirrors the ping-pong swaps and
-// writes each phase's buffers into the list.
+// and the coarse cycle of one CTA -- separated by grid barriers.  A phase runs the bodies of the level's
+// own kernels (the quad kernels', the pack's: the same arithmetic per cell) on virtual 256-thread blocks,
+// four per CTA.  The quad bodies load data written earlier in the grid through L2 (CG); the pack's load it
+// after the fences of the barrier between them.  The host mirrors the ping-pong swaps and writes each
+// phase's buffers into the list.
 enum { MP_SWEEP0 = 0, MP_SWEEP = 1, MP_RESTRICT = 2, MP_PROLONG = 3, MP_COARSE = 4 };
 constexpr int kMidLevels = 6;
 constexpr int kMidPhases = 48;
@@ -2011,12 +1674,15 @@ struct MidPhase {
     float* dst;        // sweep output / restricted right-hand side / prolongation target
     const float* src;  // sweep input / fine iterate of the restriction / coarse correction
     const float* f;    // right-hand side of the level
+    int cy;            // the level belongs to the pack: cy_*_one on 256 cells a block
 };
 struct MidPack {
     Lvl<float> L[kMidLevels];
+    CyGlobal cg[kMidLevels];
     MidPhase ph[kMidPhases];
-    LPack coarse;
-    int nph, nu1, nu2, citers, prolong;
+    CyPack pack;       // the coarse cycle's, from its level `first`
+    const float* image;
+    int first, nph, nu1, nu2, citers, prolong;
     float w;
     unsigned* bar;  // [arrivals, generation]
     int* err;
@@ -2054,14 +1720,23 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, in
     return __syncthreads_and(ok) != 0;
 }
 
-__global__ void __launch_bounds__(1024, 1) mid_cycle_kernel(MidPack P) {
-    extern __shared__ __align__(16) float lean_smem[];
+__global__ void __launch_bounds__(1024, 1) mid_cycle_kernel(const __grid_constant__ MidPack P) {
     const int sub = threadIdx.x >> 8, tid = threadIdx.x & 255;
     const int vstep = gridDim.x * 4;
     for (int k = 0; k < P.nph; ++k) {
         const MidPhase& ph = P.ph[k];
         if (ph.type == MP_COARSE) {
-            if (blockIdx.x == 0) lean_cycle(P.coarse, P.nu1, P.nu2, P.w, P.citers, P.prolong, lean_smem);
+            if (blockIdx.x == 0)
+                cy_one_cta<false>(P.pack, P.image, P.first, ph.f, ph.dst, P.nu1, P.nu2, P.w, P.citers, P.prolong);
+        } else if (ph.cy) {
+            const CyGlobal& G = P.cg[ph.level];
+            const Lvl<float>& C = P.L[ph.level + 1];
+            const int n = ph.type == MP_RESTRICT ? C.nx * C.ny * C.nz : G.n;
+            for (int i = (blockIdx.x * 4 + sub) * 256 + tid; i < n; i += vstep * 256) {
+                if (ph.type == MP_RESTRICT) cy_restrict_one<false>(ph.dst, ph.src, ph.f, G, C.nx, C.ny, i);
+                else if (ph.type == MP_PROLONG) cy_prolong_one<false>(ph.dst, ph.src, G, C.nx, C.ny, C.nz, P.prolong, i);
+                else cy_sweep_one<false>(ph.dst, nullptr, ph.src, ph.f, G, P.w, i);
+            }
         } else {
             const Lvl<float>& L = P.L[ph.level];
             const int nv = ph.gx * ph.gy;
@@ -2547,7 +2222,6 @@ struct Level {
                          // extents fit those kernels (fz_level_ok) only
     int fz_fast;      // every cell's diagonal is positive on a fully open plane with the interior z
                       // factors: the fused kernels may take their straight-line path
-    float* ccf;       // levels of at most kCoarseCells cells: per-cell stencils of the FP32 coarse cycle
     long long uni_rows; // rows flagged in uni
     double* tab64;    // per axis: glo[n], ghi[n], d[n]
     float* tab32;     // per axis: glo[n], ghi[n]
@@ -2863,7 +2537,6 @@ struct wp_mgfrac3d {
     float* r32;        // FP32 defect (right-hand side of correction cycles)
     const float* fin;  // finest right-hand side of the current solve
     const double* fin64;
-    float* ccf_all;    // the coarse levels' stencils (Level::ccf points into it)
     int tune_gen;      // bumped by every change of a level's tile or kernel variant
     // device-side cycle loop of the mixed-precision tolerance solve (see solve_mixed_graph)
     cudaGraph_t loop_graph;
@@ -2877,7 +2550,8 @@ struct wp_mgfrac3d {
     long long loop_launches[2]; // kernels of the first cycle's graph part and of one loop body
     CyPlan cy;         // the small levels' single-launch cycle (FP32): its levels are cy.l0 .. nl - 1
     int cy_from;       // levels above this one run their own kernels (wp_mgfrac3d_set_tile pins a level)
-    CyPlan cy1;        // a handle that shares the device: the levels of the pack that one CTA holds
+    CyPlan one;        // the levels of the pack that one CTA holds (see one_cta_plan)
+    int shares;        // the handle shares the device (see wp_mg_share_device)
     int fz_on;         // run the V(2,2) FP32 cycle of level 0 as the two fused kernels where it fits
     int fz_zc;         // their z planes per CTA (0 = heuristic)
     int ix_built;      // the index lists of every level exist
@@ -3006,23 +2680,6 @@ wp_status build_hierarchy(wp_mgfrac3d* h, const float* ax, const float* ay, cons
         }
     }
     h->nl = nl;
-    // per-cell stencils of the levels of at most kCoarseCells cells (a suffix of the hierarchy), in
-    // one block in level order so that any coarse-cycle pack finds its stencils contiguous
-    long cf = 0;
-    for (int l = 0; l < nl; ++l)
-        if (h->lv[l].cells <= kCoarseCells) cf += (long)kCcf * h->lv[l].cells;
-    if (cf > 0) {
-        WP_CUDA_TRY(cudaMalloc((void**)&h->ccf_all, sizeof(float) * cf));
-        long off = 0;
-        for (int l = 0; l < nl; ++l) {
-            Level& L = h->lv[l];
-            if (L.cells > kCoarseCells) continue;
-            L.ccf = h->ccf_all + off;
-            off += (long)kCcf * L.cells;
-            WP_KERNEL("cc_coeff", 40.0 * L.cells, s,
-                      cc_coeff_kernel<<<wp_cdiv(L.cells, 256), 256, 0, s>>>(L.ccf, view<float>(L)));
-        }
-    }
     return WP_OK;
 }
 
@@ -3067,6 +2724,22 @@ wp_status build_cycle_plan(wp_mgfrac3d* h, CyPlan* q, int most, cudaStream_t s) 
                       : cy_coeff_kernel<false><<<g, 256, 0, s>>>(q->image, q->pack, k, view<float>(L))));
     }
     return WP_OK;
+}
+
+// The plan of one CTA, for a handle that shares the device or runs the persistent cycle.  None for a pack whose
+// last level is divided among the CTAs: one CTA would replicate it and iterate it by other sums.  Synchronous.
+wp_status one_cta_plan(wp_mgfrac3d* h) {
+    if (h->one.image || h->cy.l0 == h->nl || h->cy.pack.lv[h->cy.pack.n - 1].P != 0) return WP_OK;
+    const wp_status st = build_cycle_plan(h, &h->one, 1, nullptr);
+    if (st != WP_OK) return st;
+    WP_CUDA_TRY(cudaStreamSynchronize(nullptr));
+    return WP_OK;
+}
+
+// level l of the pack as its global-memory kernels read it
+CyGlobal cy_global(const wp_mgfrac3d* h, int l) {
+    const CyLev& a = h->cy.pack.lv[l - h->cy.l0];
+    return CyGlobal{h->cy.image + a.cf, h->cy.pack.image, a.cap, a.nx, a.ny, a.nz, a.nxy, (int)h->lv[l].cells};
 }
 
 // the cycle from level l of the pack (see cycle_cluster_kernel)
@@ -3164,40 +2837,26 @@ wp_status smooth(Level& L, const T* f, int sweeps, T w, cudaStream_t s, bool fin
 }
 
 // The V-cycle below the finest level (from level l1, v = 0) as one mid_cycle_kernel launch when the
-// levels allow it (FP32, trilinear prolongation, nu1 >= 1, quad levels down to a lean coarse pack);
+// levels allow it (FP32, trilinear prolongation, nu1 >= 1, quad levels down to the pack);
 // sets *done.  The host mirrors every ping-pong swap the phases perform.
 wp_status mid_cycle(wp_mgfrac3d* h, int l1, int nu1, int nu2, float w, int prolong, cudaStream_t s, bool* done) {
     *done = false;
     if (!h->mid_on || h->mid_forbid || h->dims != 3 || h->mid_grid < 0 || prolong != WP_PROLONG_TRILINEAR ||
         nu1 < 1 || l1 < 1)
         return WP_OK;
-    // the coarse pack starts at the first level the fused coarse cycle takes
-    int lc = -1;
-    for (int l = l1; l < h->nl - 1 && lc < 0; ++l) {
-        long pack = 0;
-        for (int k = l; k < h->nl; ++k) pack += h->lv[k].cells;
-        if (h->lv[l].cells <= kCoarseCells && h->nl - l <= kCoarseMax && pack <= kCoarseSmemCells) lc = l;
-    }
-    if (lc <= l1 || lc - l1 + 1 > kMidLevels) return WP_OK;
-    for (int l = l1; l < lc; ++l) {
+    // quads above the pack, then the pack's levels, from level lc on in one CTA
+    const int lc = h->one.image ? h->one.l0 : -1, lq = std::min(lc, std::max(h->cy.l0, h->cy_from));
+    if (lc <= l1 || lc - l1 + 1 > kMidLevels || h->cy_from > lc) return WP_OK;
+    for (int l = l1; l < lq; ++l) {
         Level& L = h->lv[l];
         const Level& C = h->lv[l + 1];
         if (!quad_ok(L) || C.n[1] * 2 != L.n[1] || !al16(L.v) || !al16(L.t) || !al16(L.f)) return WP_OK;
     }
-    LPack Q;
-    Q.n = h->nl - lc;
-    for (int k = 0; k < Q.n; ++k) {
-        Level& E = h->lv[lc + k];
-        if (!E.ccf) return WP_OK;
-        Q.lv[k] = {E.n[0], E.n[1], E.n[2], E.ccf, E.v, E.t, E.f};
-    }
-    const size_t lean_bytes = sizeof(float) * (size_t)lean_smem_floats(Q);
-    if (lean_bytes > kLeanSmemMax) return WP_OK;
+    const size_t smem = sizeof(float) * (size_t)(h->one.pack.floats - h->one.pack.image);
     if (h->mid_grid == 0) {
         int per_sm = 0;
-        if (wp_set_smem(mid_cycle_kernel, kLeanSmemMax) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mid_cycle_kernel, 1024, kLeanSmemMax) !=
-                cudaSuccess ||
+        if (wp_set_smem(mid_cycle_kernel, smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mid_cycle_kernel, 1024, smem) != cudaSuccess ||
             per_sm < 1) {
             (void)cudaGetLastError();
             h->mid_grid = -1;
@@ -3205,9 +2864,11 @@ wp_status mid_cycle(wp_mgfrac3d* h, int l1, int nu1, int nu2, float w, int prolo
         }
         h->mid_grid = wp_sm_count();
     }
+    WP_CUDA_TRY(wp_set_smem(mid_cycle_kernel, smem));
     MidPack P;
     memset(&P, 0, sizeof(P));
     for (int l = l1; l <= lc; ++l) P.L[l - l1] = view<float>(h->lv[l]);
+    for (int l = lq; l < lc; ++l) P.cg[l - l1] = cy_global(h, l);
     auto add = [&](int type, int l, float* dst, const float* src, const float* f, int zc, int gx, int gy) {
         MidPhase& q = P.ph[P.nph++];
         q.type = type;
@@ -3218,6 +2879,7 @@ wp_status mid_cycle(wp_mgfrac3d* h, int l1, int nu1, int nu2, float w, int prolo
         q.zc = zc;
         q.gx = gx;
         q.gy = gy;
+        q.cy = l >= lq;
     };
     const int phases = (lc - l1) * (nu1 + 1 + 1 + nu2) + 1;
     if (phases > kMidPhases) return WP_OK;
@@ -3236,12 +2898,7 @@ wp_status mid_cycle(wp_mgfrac3d* h, int l1, int nu1, int nu2, float w, int prolo
         add(MP_RESTRICT, l, C.f, L.v, L.f, czc, (int)wp_cdiv((size_t)C.n[0] * (L.n[1] / 4) * 2, 256),
             (int)wp_cdiv(C.n[2], czc));
     }
-    add(MP_COARSE, lc, nullptr, nullptr, nullptr, 0, 0, 0);
-    for (int k = 0; k < Q.n; ++k) {
-        Level& E = h->lv[lc + k];
-        const int swaps = (k == Q.n - 1) ? h->coarsest_iters : nu1 + nu2;
-        if (swaps & 1) std::swap(E.v, E.t);
-    }
+    add(MP_COARSE, lc, h->lv[lc].v, nullptr, h->lv[lc].f, 0, 0, 0);
     for (int l = lc - 1; l >= l1; --l) {
         Level& L = h->lv[l];
         Level& C = h->lv[l + 1];
@@ -3252,7 +2909,9 @@ wp_status mid_cycle(wp_mgfrac3d* h, int l1, int nu1, int nu2, float w, int prolo
             std::swap(L.v, L.t);
         }
     }
-    P.coarse = Q;
+    P.pack = h->one.pack;
+    P.image = h->one.image;
+    P.first = lc - h->one.l0;
     P.nu1 = nu1;
     P.nu2 = nu2;
     P.citers = h->coarsest_iters;
@@ -3266,7 +2925,7 @@ wp_status mid_cycle(wp_mgfrac3d* h, int l1, int nu1, int nu2, float w, int prolo
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(h->mid_grid);
     cfg.blockDim = dim3(1024);
-    cfg.dynamicSmemBytes = lean_bytes;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
@@ -3320,9 +2979,10 @@ wp_status vcycle(wp_mgfrac3d* h, int l, const T* f, int nu1, int nu2, T w, int p
     }
     if constexpr (sizeof(T) == 4) {
         if (l >= h->cy.l0 && l >= h->cy_from && l < h->nl - 1) {
-            if (h->cy1.image && l < h->cy1.l0) return cy_level(h, l, f, nu1, nu2, (float)w, prolong, s, clear_v);
+            const bool split = h->shares && h->one.image;
+            if (split && l < h->one.l0) return cy_level(h, l, f, nu1, nu2, (float)w, prolong, s, clear_v);
             // the rest of the cycle in one launch of one cluster
-            const CyPlan& q = h->cy1.image ? h->cy1 : h->cy;
+            const CyPlan& q = split ? h->one : h->cy;
             double* acc = added ? acc64 : nullptr;
             cudaError_t e = cudaSuccess;
             WP_KERNEL("coarse_cycle", (double)L.cells * (3.0 * sizeof(T) + 12.0) * (nu1 + nu2 + 2), s,
@@ -3565,8 +3225,7 @@ void destroy_levels(wp_mgfrac3d* h) {
         void* ps[] = {L.tab64, L.tab32, L.fyc, L.uni, L.tuni, L.v, L.t, L.f, L.v64, L.t64, L.f64, L.imask, L.iseg};
         for (void* p : ps) if (p) cudaFree(p);
     }
-    if (h->ccf_all) cudaFree(h->ccf_all);
-    for (CyPlan* q : {&h->cy, &h->cy1})
+    for (CyPlan* q : {&h->cy, &h->one})
         if (q->image) cudaFree(q->image);
     if (h->acc) cudaFree(h->acc);
     if (h->p64) cudaFree(h->p64);
@@ -3689,8 +3348,8 @@ wp_status build_index(wp_mgfrac3d* h, cudaStream_t s) {
 wp_status cy_level(wp_mgfrac3d* h, int l, const float* f, int nu1, int nu2, float w, int prolong, cudaStream_t s, bool clear_v) {
     Level &L = h->lv[l], &C = h->lv[l + 1];
     const CyPack& P = h->cy.pack;
-    const CyLev &a = P.lv[l - h->cy.l0], &c = P.lv[l + 1 - h->cy.l0];
-    const CyGlobal G{h->cy.image + a.cf, P.image, a.cap, a.nx, a.ny, a.nz, a.nxy, (int)L.cells};
+    const CyLev& c = P.lv[l + 1 - h->cy.l0];
+    const CyGlobal G = cy_global(h, l);
     const bool d2 = h->dims == 2;
     auto sweeps = [&](int n, float wt, bool zero) {
         if (d2) launch_cy_sweeps<true>(L, G, f, n, wt, zero, s);
@@ -4206,25 +3865,29 @@ wp_status solve_mixed_loop_capture(wp_mgfrac3d* h, float* dst, const float* f, c
 // another.  A CTA only waits for phases whose tiles running CTAs hold: nothing depends on every CTA
 // being resident.  Every wait is bounded (globaltimer); a CTA that gives up raises the error flag of
 // every unfinished grid and the batch's own flag, and the other CTAs leave when they see it.
-// The per-cell arithmetic is that of the quad kernels, so a grid's iterate is the one its own
-// launch-by-launch solve produces, up to the order of the FP64 norm and mean reductions.
+// The per-cell arithmetic is that of the levels' own kernels (quads, and the pack's), so a grid's iterate
+// is the one its own launch-by-launch solve produces, up to the order of the FP64 norm and mean reductions.
 enum { PP_INIT = 0, PP_DEFECT, PP_SWEEP0, PP_SWEEP, PP_SWEEP_ACC, PP_RESTRICT, PP_PROLONG, PP_COARSE, PP_CONVERT };
 enum { PT_NONE = 0, PT_START = 1, PT_STEP = 2 };
 
 struct PPhase {
     int type, level, zc, gx;
     int nvb, per, ntiles, test;  // 256-thread blocks, blocks per tile (a multiple of 4), tiles, stopping rule
-    int cnx, cny, cnz, pack;     // coarse level extents (restriction, prolongation); coarse pack index
+    int cnx, cny, cnz;           // coarse level extents (restriction, prolongation)
+    int cy;                      // the level belongs to the pack: cy_*_one on 256 cells a block (coarse cycle: its
+                                 // last level's sweeps alone, from global memory)
     float* dst;
     const float* src;
     const float* f;
+    CyGlobal cg;
 };
 
 struct PGrid {
     Lvl<float> L[kMaxLevels];
     Lvl<double> L0;        // FP64 view of the finest level
     const PPhase* ph;
-    const LPack* packs;
+    const CyPack* pack;    // the coarse cycle's, from its level `first`
+    const float* image;
     MgLoop* loop;          // the handle's loop state (cycles, steps, relative residual history)
     double* acc;           // the handle's slots: ||r||^2, ||f||^2, sum of f over active cells, their count
     int* err;              // the handle's device error flag
@@ -4232,7 +3895,7 @@ struct PGrid {
     float* r32;
     const float* f;        // finest right-hand side
     float* dst;            // FP32 copy of the solution
-    int nph, loop_pc, end_pc, nu1, nu2, citers, prolong;
+    int nph, loop_pc, end_pc, nu1, nu2, citers, prolong, first, d2;
     float w;
 };
 
@@ -4427,8 +4090,36 @@ __device__ __noinline__ void pb_prolong(const PPhase& Ps, const Lvl<float>& Ls, 
     for (int vb = vb0; vb < v1; vb += 4)
         prolong_tri_q_body<float, kPbCG>(P.dst, P.src, L.nx, L.ny, L.nz, P.cnx, P.cny, P.cnz, vb % P.gx, vb / P.gx, tid);
 }
-__device__ __noinline__ void pb_coarse(const LPack& Q, const PGrid& G, float* lean_smem) {
-    lean_cycle<true>(Q, G.nu1, G.nu2, G.w, G.citers, G.prolong, lean_smem);
+// the same phases of a level of the pack, 256 cells a block
+template <bool D2>
+__device__ __noinline__ void pb_cy(const PPhase& Ps, float w, double* p64, int prolong, int vb0, int v1, int tid) {
+    const PPhase P = Ps;
+    const int n = P.type == PP_RESTRICT ? P.cnx * P.cny * P.cnz : P.cg.n;
+    for (int vb = vb0; vb < v1; vb += 4) {
+        const int i = vb * 256 + tid;
+        if (i >= n) break;
+        if (P.type == PP_RESTRICT) cy_restrict_one<D2>(P.dst, P.src, P.f, P.cg, P.cnx, P.cny, i);
+        else if (P.type == PP_PROLONG) cy_prolong_one<D2>(P.dst, P.src, P.cg, P.cnx, P.cny, P.cnz, prolong, i);
+        else cy_sweep_one<D2>(P.dst, P.type == PP_SWEEP_ACC ? p64 : nullptr, P.src, P.f, P.cg, w, i);
+    }
+}
+// the last level's sweeps from zero by one CTA, between dst (written first) and src
+template <bool D2>
+__device__ __noinline__ void pb_cy_last(const PPhase& Ps, float w, int citers) {
+    const PPhase P = Ps;
+    float *to = P.dst, *from = const_cast<float*>(P.src);
+    for (int k = 0; k < citers; ++k) {
+        for (int i = threadIdx.x; i < P.cg.n; i += 1024) cy_sweep_one<D2>(to, nullptr, k ? from : nullptr, P.f, P.cg, w, i);
+        __syncthreads();
+        float* u = to;
+        to = from;
+        from = u;
+    }
+}
+template <bool D2>
+__device__ __forceinline__ void pb_coarse(const PPhase& P, const PGrid& G) {
+    if (P.cy) pb_cy_last<D2>(P, G.w, G.citers);
+    else cy_one_cta<D2>(*G.pack, G.image, G.first, P.f, P.dst, G.nu1, G.nu2, G.w, G.citers, G.prolong);
 }
 // active-cell sum and count of f (active_sum_q_kernel), ||f||^2 (sumsq_kernel), p64 = 0
 __device__ __noinline__ void pb_init(const PPhase& Ps, const Lvl<double>& Ls, const float* f, double* p64, int vb0,
@@ -4473,7 +4164,6 @@ __device__ __noinline__ double pb_defect(const PPhase& Ps, const Lvl<double>& Ls
 }
 
 __global__ void __launch_bounds__(1024, 1) batch_persist_kernel(PArgs A) {
-    extern __shared__ __align__(16) float lean_smem[];
     __shared__ Lvl<float> sL;
     __shared__ Lvl<double> sD;
     __shared__ PPhase sP;
@@ -4536,8 +4226,14 @@ __global__ void __launch_bounds__(1024, 1) batch_persist_kernel(PArgs A) {
         if (prof && threadIdx.x == 0) c2 = clock64();
         const int type = sP.type;
         const int vb0 = sP.per * t + sub, v1 = min(sP.per * (t + 1), sP.nvb);
-        switch (type) {
-            case PP_COARSE: pb_coarse(G.packs[sP.pack], G, lean_smem); break;
+        if (sP.cy && type != PP_COARSE) {
+            if (G.d2) pb_cy<true>(sP, G.w, G.p64, G.prolong, vb0, v1, tid);
+            else pb_cy<false>(sP, G.w, G.p64, G.prolong, vb0, v1, tid);
+        } else switch (type) {
+            case PP_COARSE:
+                if (G.d2) pb_coarse<true>(sP, G);
+                else pb_coarse<false>(sP, G);
+                break;
             case PP_INIT: {
                 double o[3];
                 pb_init(sP, sD, G.f, G.p64, vb0, v1, tid, o);
@@ -4594,16 +4290,15 @@ void pp_tiles(PPhase& q, long nvb, long cells_vb, long target) {
     q.ntiles = (int)std::max(1L, nt);
 }
 
-// One grid's program (PGrid's phases and coarse packs), built by mirroring the buffer swaps of the
+// One grid's program (PGrid's phases), built by mirroring the buffer swaps of the
 // launch-by-launch cycle on copies of the level pointers (the handle is not changed).
 struct PBuild {
     wp_mgfrac3d* h;
-    int nu1, nu2, lc;
+    int nu1, nu2, lc;  // lc: first level of the one-CTA coarse cycle (the number of levels: none)
     long target;
     float* v[kMaxLevels];
     float* t[kMaxLevels];
     std::vector<PPhase> ph;
-    std::vector<LPack> packs;
 
     PPhase base(int type, int l) const {
         PPhase q;
@@ -4625,38 +4320,46 @@ struct PBuild {
         ph.push_back(q);
     }
     void cycle(int l, const float* f, bool clear, bool acc) {
-        if (l == lc) {
-            LPack Q;
-            memset(&Q, 0, sizeof(Q));
-            Q.n = h->nl - lc;
-            for (int k = 0; k < Q.n; ++k) {
-                Level& E = h->lv[lc + k];
-                Q.lv[k] = {E.n[0], E.n[1], E.n[2], E.ccf, v[lc + k], t[lc + k], E.f};
-            }
+        const bool pack = l >= h->cy.l0;
+        if (l == lc || l == h->nl - 1) {
             PPhase q = base(PP_COARSE, l);
-            q.pack = (int)packs.size();
             q.nvb = q.per = q.ntiles = 1;
-            packs.push_back(Q);
-            ph.push_back(q);
-            for (int k = 0; k < Q.n; ++k) {
-                const int swaps = (k == Q.n - 1) ? h->coarsest_iters : nu1 + nu2;
-                if (swaps & 1) std::swap(v[lc + k], t[lc + k]);
+            q.dst = v[l];
+            q.f = f;
+            if (l != lc) {
+                q.cy = 1;
+                q.cg = cy_global(h, l);
+                q.dst = t[l];
+                q.src = v[l];
+                if (h->coarsest_iters & 1) std::swap(v[l], t[l]);
             }
+            ph.push_back(q);
             return;
         }
         const Level& L = h->lv[l];
         const Level& C = h->lv[l + 1];
         const int zc = zc_of(L);
         const long gx = quads(L);
+        // a phase over `cells` cells of the pack, else over nvb quad blocks.  The pack counts a 2D level's
+        // extents its own way (CyLev).
+        auto tiles = [&](PPhase& q, long cells, long nvb, long cells_vb) {
+            const CyLev* c = pack ? &h->cy.pack.lv[l + 1 - h->cy.l0] : nullptr;
+            q.cy = pack;
+            if (pack) q.cg = cy_global(h, l);
+            q.cnx = pack ? c->nx : C.n[0];
+            q.cny = pack ? c->ny : C.n[1];
+            q.cnz = pack ? c->nz : C.n[2];
+            pp_tiles(q, pack ? (long)wp_cdiv(cells, 256) : nvb, pack ? 256 : cells_vb, target);
+            ph.push_back(q);
+        };
         auto sweep = [&](int type) {
             PPhase q = base(type, l);
             q.zc = zc;
             q.gx = (int)gx;
             q.dst = type == PP_SWEEP_ACC ? nullptr : t[l];
-            q.src = v[l];
+            q.src = type == PP_SWEEP0 ? nullptr : v[l];
             q.f = f;
-            pp_tiles(q, gx * (long)wp_cdiv(L.n[2], zc), 1024L * zc, target);
-            ph.push_back(q);
+            tiles(q, L.cells, gx * (long)wp_cdiv(L.n[2], zc), 1024L * zc);
             std::swap(v[l], t[l]);
         };
         int pre = nu1;
@@ -4673,11 +4376,7 @@ struct PBuild {
             q.dst = C.f;
             q.src = v[l];
             q.f = f;
-            q.cnx = C.n[0];
-            q.cny = C.n[1];
-            q.cnz = C.n[2];
-            pp_tiles(q, q.gx * (long)wp_cdiv(C.n[2], czc), 2048L * czc, target);
-            ph.push_back(q);
+            tiles(q, C.cells, q.gx * (long)wp_cdiv(C.n[2], czc), 2048L * czc);
         }
         cycle(l + 1, C.f, true, false);
         {
@@ -4685,21 +4384,18 @@ struct PBuild {
             q.gx = (int)gx;
             q.dst = v[l];
             q.src = v[l + 1];
-            q.cnx = C.n[0];
-            q.cny = C.n[1];
-            q.cnz = C.n[2];
-            pp_tiles(q, gx * (long)L.n[2], 1024L, target);
-            ph.push_back(q);
+            tiles(q, L.cells, gx * (long)L.n[2], 1024L);
         }
         for (int k = 0; k < nu2; ++k) sweep(acc && k == nu2 - 1 ? PP_SWEEP_ACC : PP_SWEEP);
     }
 };
 
-// Whether handle h can run its mixed solve as a persistent program (quad levels with aligned work
-// arrays down to a lean coarse pack that fits the CTA's shared memory): the pack's first level, its
-// shared bytes, or -1 with a message.
-int persist_plan(wp_mgfrac3d* h, const wp_mg_params* prm, size_t smem_cap, size_t* lean_bytes, const char** why) {
+// Whether handle h, which shares the device, can run its mixed solve as a persistent program (quad levels with
+// aligned work arrays down to a coarse level of at most 4096 cells): the first level of the one-CTA coarse
+// cycle (the number of levels where the pack has none), its shared bytes, or -1 with a message.
+int persist_plan(wp_mgfrac3d* h, const wp_mg_params* prm, size_t smem_cap, size_t* bytes, const char** why) {
     *why = nullptr;
+    *bytes = 0;
     if (prm->prolongation != WP_PROLONG_TRILINEAR || prm->nu1 < 1 || prm->nu2 < 1 || prm->start == WP_START_FMG) {
         *why = "the persistent batch runs trilinear V(nu1, nu2) cycles with nu1, nu2 >= 1 from a zero start";
         return -1;
@@ -4727,28 +4423,23 @@ int persist_plan(wp_mgfrac3d* h, const wp_mg_params* prm, size_t smem_cap, size_
             return -1;
         }
     }
-    LPack Q;
-    Q.n = h->nl - lc;
-    for (int k = 0; k < Q.n; ++k) {
-        const Level& E = h->lv[lc + k];
-        if (!E.ccf) {
-            *why = "a coarse level has no precomputed stencils";
-            return -1;
-        }
-        Q.lv[k] = {E.n[0], E.n[1], E.n[2], E.ccf, E.v, E.t, E.f};
+    if (h->cy.l0 == h->nl) {
+        *why = "a grid's small levels do not fit the shared memory of a cluster";
+        return -1;
     }
-    *lean_bytes = sizeof(float) * (size_t)lean_smem_floats(Q, true);
-    if (*lean_bytes > smem_cap) {
+    if (!h->one.image) return h->nl;
+    *bytes = sizeof(float) * (size_t)(h->one.pack.floats - h->one.pack.image);
+    if (*bytes > smem_cap) {
         *why = "a grid's coarse pack does not fit the persistent CTA's shared memory";
         return -1;
     }
-    return lc;
+    return std::max(1, h->one.l0);
 }
 
-// Builds handle h's program into ph / packs and fills its descriptor (device pointers of the
-// program arrays are set by the caller).
+// Builds handle h's program into ph and fills its descriptor (device pointers of the program arrays are
+// set by the caller).
 void persist_program(wp_mgfrac3d* h, const wp_mg_params* prm, float* dst, const float* f, long target, int lc,
-                     PGrid* G, std::vector<PPhase>& ph, std::vector<LPack>& packs) {
+                     PGrid* G, std::vector<PPhase>& ph) {
     PBuild b;
     b.h = h;
     b.nu1 = prm->nu1;
@@ -4772,7 +4463,10 @@ void persist_program(wp_mgfrac3d* h, const wp_mg_params* prm, float* dst, const 
         b.ph.push_back(q);
     }
     memset(G, 0, sizeof(*G));
-    for (int l = 0; l <= lc; ++l) G->L[l] = view<float>(h->lv[l]);
+    for (int l = 0; l < h->nl; ++l) G->L[l] = view<float>(h->lv[l]);
+    G->image = h->one.image;
+    G->first = lc - h->one.l0;
+    G->d2 = h->dims == 2;
     G->L0 = view<double>(h->lv[0]);
     G->loop = reinterpret_cast<MgLoop*>(h->loop_state);
     G->acc = h->acc;
@@ -4790,7 +4484,6 @@ void persist_program(wp_mgfrac3d* h, const wp_mg_params* prm, float* dst, const 
     G->prolong = prm->prolongation;
     G->w = (float)prm->omega;
     ph.swap(b.ph);
-    packs.swap(b.packs);
 }
 
 }  // namespace
@@ -4804,7 +4497,7 @@ struct wp_mg_pbatch {
     PCtl* d_ctl = nullptr;
     PCtl ctl{-1, 0, 0};         // the control block's value on the device
     unsigned long long* d_prof = nullptr;  // kProfSlots counters (see PCtl::prof)
-    std::vector<void*> blobs;   // per grid: phases, then coarse packs
+    std::vector<void*> blobs;   // per grid: phases, then the coarse cycle's pack
     size_t smem = 0;
     int grid = 0;
     wp_mg_params prm;
@@ -4850,21 +4543,20 @@ wp_status wp_mg_pbatch_create(wp_mg_pbatch** out, wp_mgfrac3d* const* hs, float*
     std::vector<PGrid> G(count);
     wp_status st = WP_OK;
     for (int i = 0; i < count && st == WP_OK; ++i) {
-        size_t lean = 0;
+        size_t bytes = 0;
         const char* why = nullptr;
-        const int lc = persist_plan(hs[i], prm, cap, &lean, &why);
+        const int lc = persist_plan(hs[i], prm, cap, &bytes, &why);
         if (lc < 0) {
             wp_set_error_msg(why);
             st = WP_ERR_UNSUPPORTED;
             break;
         }
-        pb->smem = std::max(pb->smem, lean);
+        pb->smem = std::max(pb->smem, bytes);
         std::vector<PPhase> ph;
-        std::vector<LPack> packs;
-        persist_program(hs[i], prm, dst[i], f[i], pb->target, lc, &G[i], ph, packs);
+        persist_program(hs[i], prm, dst[i], f[i], pb->target, lc, &G[i], ph);
         hs[i]->last64 = 1;  // the FP64 iterate of the last solve is p64
         for (const PPhase& q : ph) pb->tiles += q.ntiles;
-        const size_t bph = sizeof(PPhase) * ph.size(), bpk = sizeof(LPack) * packs.size();
+        const size_t bph = sizeof(PPhase) * ph.size(), bpk = sizeof(CyPack);
         const size_t off = (bph + 255) / 256 * 256;
         void* blob = nullptr;
         cudaError_t e = cudaMalloc(&blob, off + bpk + 16);
@@ -4872,14 +4564,14 @@ wp_status wp_mg_pbatch_create(wp_mg_pbatch** out, wp_mgfrac3d* const* hs, float*
             pb->blobs.push_back(blob);
             e = cudaMemcpy(blob, ph.data(), bph, cudaMemcpyHostToDevice);
         }
-        if (e == cudaSuccess && bpk) e = cudaMemcpy((char*)blob + off, packs.data(), bpk, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy((char*)blob + off, &hs[i]->one.pack, bpk, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
             wp_set_cuda_error(e, "persistent batch programs", __FILE__, __LINE__);
             st = WP_ERR_CUDA;
             break;
         }
         G[i].ph = reinterpret_cast<const PPhase*>(blob);
-        G[i].packs = reinterpret_cast<const LPack*>((char*)blob + off);
+        G[i].pack = reinterpret_cast<const CyPack*>((char*)blob + off);
     }
     if (st == WP_OK) {
         cudaError_t e = cudaMalloc((void**)&pb->d_grids, sizeof(PGrid) * count);
@@ -5247,7 +4939,8 @@ wp_status autotune(wp_mgfrac3d* h, cudaStream_t s) {
     }
     // the levels below the finest as one persistent launch, or launch by launch: time a V-cycle from
     // level 1 both ways (the levels are L2-resident: no flush) and keep the faster
-    if (st == WP_OK && h->dims == 3 && h->nl >= 3 && !h->mid_forbid && h->cy.l0 > 1) {
+    if (st == WP_OK && h->dims == 3 && h->nl >= 3 && !h->mid_forbid && h->cy.l0 > 1 &&
+        (st = one_cta_plan(h)) == WP_OK) {
         float best = 1e30f;
         int best_on = 1;
         for (int on = 1; on >= 0 && st == WP_OK; --on) {
@@ -5268,7 +4961,7 @@ wp_status autotune(wp_mgfrac3d* h, cudaStream_t s) {
     // adds into an FP64 iterate -- here a scratch array, not the handle's), after an L2 flush when
     // level 0 exceeds it; the fused passes only when they are clearly (5%) faster -- at 256^3 the
     // two measure alike and the one-sweep kernels use the memory bandwidth better per byte
-    if (st == WP_OK && h->dims == 3 && h->nl >= 2 && h->lv[0].tuni && h->cy.l0 > 0) {
+    if (st == WP_OK && h->dims == 3 && h->nl >= 2 && h->lv[0].tuni && h->cy.l0 > 0 && !h->shares) {
         Level& L0 = h->lv[0];
         double* acc = nullptr;
         if (cudaMalloc((void**)&acc, sizeof(double) * L0.cells) != cudaSuccess) {
@@ -5333,6 +5026,10 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_tiles(const wp_mgfrac3d* h, int* zc,
 extern "C" CUWHHD_API wp_status wp_mgfrac3d_set_tile(wp_mgfrac3d* h, int level, int kind, int zc, int variant) {
     if (h && kind == 3 && (variant == 0 || variant == 1)) {
         // the levels below the finest: one persistent launch (1) or launch by launch (0)
+        if (variant && h->dims == 3) {
+            const wp_status st = one_cta_plan(h);
+            if (st != WP_OK) return st;
+        }
         h->mid_on = variant;
         ++h->tune_gen;
         return WP_OK;
@@ -5372,18 +5069,17 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_uniform_rows(const wp_mgfrac3d* h, i
 }
 
 wp_status wp_mg_prepare_mixed(wp_mgfrac3d* h) { return prepare_mixed(h); }
-// For the batch, whose grids run on concurrent graph branches.  A cooperative launch needs the whole GPU, so
+// For the batch, whose grids run on concurrent graph branches, or as phases of the persistent kernel with the
+// same bits: so its level 0 never takes the fused pair (the tuner has not preferred it for any grid).  A cooperative launch needs the whole GPU, so
 // the levels go launch by launch, and of the pack only those that one CTA holds share a launch: a cluster of 16
 // is faster for one grid and dearer for many (16 SMs for 31 to 50 us a cycle: 64 uneven 2D and 3D grids took
 // 31.4 ms with it, 28.6 before).  The pack's larger levels keep its arithmetic, so that a grid's results are those
 // of its own solver; a pack whose last level is divided among the CTAs is kept whole.
 wp_status wp_mg_share_device(wp_mgfrac3d* h) {
     h->mid_forbid = 1;
-    if (h->cy.l0 == h->nl || h->cy.pack.lv[h->cy.pack.n - 1].P != 0) return WP_OK;
-    const wp_status st = build_cycle_plan(h, &h->cy1, 1, nullptr);
-    if (st != WP_OK) return st;
-    WP_CUDA_TRY(cudaStreamSynchronize(nullptr));
-    return WP_OK;
+    h->shares = 1;
+    h->fz_on = 0;
+    return one_cta_plan(h);
 }
 wp_status wp_mg_solve_mixed_loop_capture(wp_mgfrac3d* h, float* dst, const float* f, const wp_mg_params* prm,
                                          cudaStream_t s, long long* body_launches) {

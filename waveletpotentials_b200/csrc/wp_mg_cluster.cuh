@@ -16,10 +16,14 @@
 // A 2D level (nx, ny) is the slab problem (1, ny, nx): planes are rows along y.
 //
 // A handle that shares the device takes only the levels of one CTA this way, and the pack's larger levels by
-// the kernels at the end of this file (see wp_mg_share_device).
+// the kernels at the end of this file (see wp_mg_share_device); the persistent cycle and the persistent batch
+// run the same two halves as phases of theirs.  All of them give the same bits.
 // Measured (B200, per V(2,2) cycle): 32^3 ... 2^3 31 us in one launch, formerly 75 us in six; 2D 256^2 ... 2^2 50 us
 // against 110 us.  Projections: 32^3 872 -> 663 us, 128^3 (FP32) 2292 -> 2000 us, 2D 256^2 1055 -> 731 us.
+// The cycle's functions have two forms, CL: the cluster's CTAs of 512 threads, stencils in shared memory; else one
+// 1024-thread CTA of a persistent kernel, stencils read through L1, which the kernel's other work needs large.
 constexpr int kCyThreads = 512;
+__host__ __device__ constexpr int cy_nt(bool cl) { return cl ? kCyThreads : 1024; }
 constexpr int kCyMax = 12;           // levels of a pack
 constexpr int kCyCells = 4096;       // cells of a level a CTA may hold
 // floats per cell: the face coefficients y- y+ z- z+ and (3D) x- x+, then 1 / diagonal (0: inactive) and
@@ -119,11 +123,14 @@ struct CySm {
     int lo, hi;         // a neighbour owns the planes below / above
     unsigned mxy, my;   // i / nxy = umulhi(i, mxy), rem / ny = umulhi(rem, my) (0: a divisor of 1)
     int cf, f, v, t;
+    const float* gcf;   // without CL: the stencils
 };
 constexpr int kCyHead = 256; // floats reserved for the level table
 static_assert(kCyMax * sizeof(CySm) <= kCyHead * sizeof(float), "level table");
 extern __shared__ __align__(16) float cy_smem[];
 __device__ __forceinline__ const CySm& cy_lv(int l) { return reinterpret_cast<const CySm*>(cy_smem)[l]; }
+template <bool CL>
+__device__ __forceinline__ const float* cy_stencils(const CySm& S) { return CL ? cy_smem + S.cf : S.gcf; }
 __device__ __forceinline__ int cy_div(int i, unsigned m) { return m ? (int)__umulhi((unsigned)i, m) : i; }
 
 // The passes below are calls, not inlined: a cycle runs each of them once or a few times per level, so its time
@@ -133,6 +140,7 @@ __device__ __forceinline__ int cy_div(int i, unsigned m) { return m ? (int)__umu
 // Copies the neighbours' planes beside this CTA's into the halos of b (a buffer every CTA has finished
 // writing).  A remote load instruction takes the SM some 40 cycles whatever its width, so planes move 16
 // bytes per lane: reading them word by word inside the sweeps made a 32^3 sweep 3600 cycles.
+template <bool CL>
 __device__ __noinline__ void cy_halos(int l, int bo, int rank) {
     const CySm& S = cy_lv(l);
     const int nxy = S.nxy, cap = S.cap;
@@ -140,7 +148,7 @@ __device__ __noinline__ void cy_halos(int l, int bo, int rank) {
     float* b = cy_smem + bo;
     if (((nxy | bo) & 3) == 0) {
 #pragma unroll 1
-        for (int i = 4 * threadIdx.x; i < 2 * nxy; i += 4 * kCyThreads) {
+        for (int i = 4 * threadIdx.x; i < 2 * nxy; i += 4 * cy_nt(CL)) {
             const bool up = i >= nxy;
             const int j = up ? i - nxy : i;
             if (up ? hi : lo)
@@ -149,7 +157,7 @@ __device__ __noinline__ void cy_halos(int l, int bo, int rank) {
         }
     } else {
 #pragma unroll 1
-        for (int i = threadIdx.x; i < 2 * nxy; i += kCyThreads) {
+        for (int i = threadIdx.x; i < 2 * nxy; i += cy_nt(CL)) {
             const bool up = i >= nxy;
             const int j = up ? i - nxy : i;
             if (up ? hi : lo) b[up ? cap + j : j - nxy] = up ? cy_pull(b + j, rank + 1) : cy_pull(b + cap - nxy + j, rank - 1);
@@ -211,27 +219,27 @@ __device__ __forceinline__ float cy_interp(const float* u, int x, int y, int z, 
 // One pass over the owned cells: CY_SWEEP dst = src + w (f - A src) / diagonal (0 where the diagonal is 0; from
 // zero if so < 0), CY_RESID dst = the residual times the restriction weight.  Ends with every CTA in
 // step (CY_SWEEP) or this one (CY_RESID).
-template <bool D2>
+template <bool D2, bool CL>
 __device__ __noinline__ void cy_pass(int l, int so, int dof, float w, int mode, int rank) {
     const CySm& S = cy_lv(l);
     const int cap = S.cap, nxy = S.nxy, ny = S.ny, n = S.n, P = S.P;
-    const float *cf = cy_smem + S.cf, *f = cy_smem + S.f, *src = cy_smem + so;
+    const float *cf = cy_stencils<CL>(S), *f = cy_smem + S.f, *src = cy_smem + so;
     float* dst = cy_smem + dof;
-    if (so >= 0 && P) cy_halos(l, so, rank);
+    if (so >= 0 && P) cy_halos<CL>(l, so, rank);
 #pragma unroll 2
-    for (int i = threadIdx.x; i < n; i += kCyThreads)
+    for (int i = threadIdx.x; i < n; i += cy_nt(CL))
         dst[i] = cy_cell<D2>(cf + i, cap, ny, nxy, f[i], w, mode, so < 0, [src, i](int o) { return src[i + o]; });
     if (mode == CY_SWEEP && P) cy_barrier();
     else __syncthreads();
 }
 
 // n sweeps of v (from zero: zero); v the iterate's offset, t the other buffer's
-template <bool D2>
+template <bool D2, bool CL>
 __device__ __forceinline__ void cy_smooth(int l, int& v, int& t, int n, float w, bool zero, int rank) {
-    if (zero && n == 0) cy_pass<D2>(l, -1, v, 0.f, CY_SWEEP, rank);
+    if (zero && n == 0) cy_pass<D2, CL>(l, -1, v, 0.f, CY_SWEEP, rank);
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
-        cy_pass<D2>(l, zero && k == 0 ? -1 : v, t, w, CY_SWEEP, rank);
+        cy_pass<D2, CL>(l, zero && k == 0 ? -1 : v, t, w, CY_SWEEP, rank);
         const int u = v;
         v = t;
         t = u;
@@ -239,7 +247,7 @@ __device__ __forceinline__ void cy_smooth(int l, int& v, int& t, int n, float w,
 }
 
 // f of level l + 1 = the sums of level l's weighted residuals r over each coarse cell's children
-template <bool D2>
+template <bool D2, bool CL>
 __device__ __noinline__ void cy_sums(int l, int ro) {
     const CySm *S = &cy_lv(l), *C = &cy_lv(l + 1);
     float *r = cy_smem + ro, *fc = cy_smem + C->f;
@@ -250,7 +258,7 @@ __device__ __noinline__ void cy_sums(int l, int ro) {
     const bool gather = S->P && C->P == 0;
     float* out = gather ? r + S->cap : fc;
 #pragma unroll 1
-    for (int i = threadIdx.x; i < (planes ? cz1 - cz0 : 0) * cnxy; i += kCyThreads) {
+    for (int i = threadIdx.x; i < (planes ? cz1 - cz0 : 0) * cnxy; i += cy_nt(CL)) {
         const int pz = cy_div(i, C->mxy), rem = i - pz * cnxy, x = D2 ? 0 : cy_div(rem, C->my), y = rem - x * C->ny;
         float s = 0.f;
 #pragma unroll 1
@@ -269,7 +277,7 @@ __device__ __noinline__ void cy_sums(int l, int ro) {
     if (gather) {
         cy_barrier();
 #pragma unroll 1
-        for (int i = threadIdx.x; i < C->cap; i += kCyThreads) {
+        for (int i = threadIdx.x; i < C->cap; i += cy_nt(CL)) {
             const int z = cy_div(i, C->mxy), rem = i - z * cnxy;
             float s = cy_pull(out + rem, 2 * z);
             if (2 * z + 1 < S->nz) s += cy_pull(out + rem, 2 * z + 1);
@@ -280,16 +288,16 @@ __device__ __noinline__ void cy_sums(int l, int ro) {
 }
 
 // v += P vc, v of level l, vc of level l + 1
-template <bool D2>
+template <bool D2, bool CL>
 __device__ __noinline__ void cy_prolong(int l, int vo, int vco, int kind, int rank) {
     const CySm *S = &cy_lv(l), *C = &cy_lv(l + 1);
     float* v = cy_smem + vo;
     const int cnxy = C->nxy, cny = C->ny, cnx = C->nx, cnz = C->nz;
-    if (S->P && C->P) cy_halos(l + 1, vco, rank);
+    if (S->P && C->P) cy_halos<CL>(l + 1, vco, rank);
     const int base = vco - C->z0 * cnxy;
     const int nxy = S->nxy, ny = S->ny, z0 = S->z0, n = S->n;
 #pragma unroll 2
-    for (int i = threadIdx.x; i < n; i += kCyThreads) {
+    for (int i = threadIdx.x; i < n; i += cy_nt(CL)) {
         const int pz = cy_div(i, S->mxy), rem = i - pz * nxy, x = D2 ? 0 : cy_div(rem, S->my), y = rem - x * ny;
         v[i] += cy_interp<D2>(cy_smem + base, x, y, z0 + pz, cnx, cny, cnz, kind);
     }
@@ -301,12 +309,12 @@ __device__ __noinline__ void cy_prolong(int l, int vo, int vco, int kind, int ra
 // zero are one linear map of f.  One warp forms it (row i, column j at m[8 i + j]) in the prologue, while
 // the previous kernel still runs, by sweeping the unit right-hand sides: lane l carries cell l & 7 of the
 // columns 2 (l >> 3) and 2 (l >> 3) + 1.
-template <bool D2>
+template <bool D2, bool CL>
 __device__ __noinline__ void cy_coarsest_map(int l, float* m, float w, int citers) {
     constexpr int NC = cy_floats(D2) - 2;
     const CySm* S = &cy_lv(l);
     const int lane = threadIdx.x, i = lane & 7, cap = S->cap;
-    const float* cf = cy_smem + S->cf;
+    const float* cf = cy_stencils<CL>(*S);
     const int step[3] = {1, S->nxy, S->ny};
     const float rd = i < cap ? cf[NC * cap + i] : 0.f;
     float c[3] = {0.f, 0.f, 0.f};
@@ -341,12 +349,12 @@ __device__ __noinline__ void cy_coarsest_map(int l, float* m, float w, int citer
 }
 
 // citers sweeps from zero of a replicated level of at most 32 cells by one warp, a cell per lane in registers
-template <bool D2>
+template <bool D2, bool CL>
 __device__ __noinline__ void cy_warp_sweeps(int l, float* v, float w, int citers) {
     constexpr int NC = cy_floats(D2) - 2;
     const CySm* S = &cy_lv(l);
     const int n = S->cap, i = threadIdx.x;
-    const float *cf = cy_smem + S->cf, *f = cy_smem + S->f;
+    const float *cf = cy_stencils<CL>(*S), *f = cy_smem + S->f;
     const int off[6] = {-1, 1, -S->nxy, S->nxy, -S->ny, S->ny};
     const float rd = i < n ? cf[NC * n + i] : 0.f;
     float c[NC], x = 0.f;
@@ -373,24 +381,20 @@ __device__ __noinline__ void cy_warp_sweeps(int l, float* v, float w, int citers
 }
 
 // V-cycle from level `first` of the pack: f the level's right-hand side, from v = 0 or (vin) from vin,
-// into vout or (p64) added to p64.
-template <bool D2>
-__global__ void __launch_bounds__(kCyThreads) cycle_cluster_kernel(const __grid_constant__ CyPack C,
-                                                                   const float* __restrict__ image, int first,
-                                                                   const float* f, const float* vin, float* vout,
-                                                                   double* p64, int nu1, int nu2, float w, int citers,
-                                                                   int prolong) {
+// into vout or (p64) added to p64.  What the previous kernel wrote is first read after wp_pdl_enter.
+template <bool D2, bool CL>
+__device__ __forceinline__ void cy_cycle(const CyPack& C, const float* image, int rank, int first, const float* f,
+                                         const float* vin, float* vout, double* p64, int nu1, int nu2, float w, int citers,
+                                         int prolong) {
     __shared__ float cmap[64];
     float* sm = cy_smem;
     CySm* S = reinterpret_cast<CySm*>(cy_smem);
-    uint32_t rank_u;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank_u));
-    const int rank = (int)rank_u, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     // the stencils are constant: their copy starts before the previous kernel has finished
-    {
+    if (CL) {
         const float* g = image + (long)rank * C.image;
         const int from = C.lv[first].cf;  // a multiple of 4
-        for (int i = from / 4 + tid; i < C.image / 4; i += kCyThreads) cp_async16(sm + kCyHead + 4 * i, g + 4 * i);
+        for (int i = from / 4 + tid; i < C.image / 4; i += cy_nt(CL)) cp_async16(sm + kCyHead + 4 * i, g + 4 * i);
         cp_async_commit();
     }
     if (tid < C.n) {
@@ -405,7 +409,9 @@ __global__ void __launch_bounds__(kCyThreads) cycle_cluster_kernel(const __grid_
         // exact for the indices here: i d < 2^32 (at most 2^13 cells)
         q.mxy = L.nxy > 1 ? (unsigned)((0x100000000ull + L.nxy - 1) / L.nxy) : 0u;
         q.my = L.ny > 1 ? (unsigned)((0x100000000ull + L.ny - 1) / L.ny) : 0u;
-        q.cf = kCyHead + L.cf; q.f = kCyHead + L.f; q.v = kCyHead + L.v; q.t = kCyHead + L.t;
+        const int at = CL ? kCyHead : kCyHead - C.image;
+        q.cf = at + L.cf; q.f = at + L.f; q.v = at + L.v; q.t = at + L.t;
+        q.gcf = image + L.cf;
         S[tid] = q;
     }
     __syncthreads();
@@ -414,7 +420,7 @@ __global__ void __launch_bounds__(kCyThreads) cycle_cluster_kernel(const __grid_
     for (int l = first; l < C.n; ++l) {
         const CySm& q = S[l];
 #pragma unroll 1
-        for (int i = tid; i < 2 * q.nxy + q.cap - q.n; i += kCyThreads) {
+        for (int i = tid; i < 2 * q.nxy + q.cap - q.n; i += cy_nt(CL)) {
             const int j = i < q.nxy ? i - q.nxy : q.n + i - q.nxy;
             sm[q.v + j] = 0.f;
             sm[q.t + j] = 0.f;
@@ -424,12 +430,12 @@ __global__ void __launch_bounds__(kCyThreads) cycle_cluster_kernel(const __grid_
     const bool mapped = C.lv[last].P == 0 && C.lv[last].nx <= 2 && C.lv[last].ny <= 2 && C.lv[last].nz <= 2;
     cp_async_wait<0>();
     __syncthreads();
-    if (mapped && tid < 32) cy_coarsest_map<D2>(last, cmap, w, citers);
-    wp_pdl_enter();
+    if (mapped && tid < 32) cy_coarsest_map<D2, CL>(last, cmap, w, citers);
+    if (CL) wp_pdl_enter();
     const CySm& F = S[first];
     const long g0 = (long)F.z0 * F.nxy;
 #pragma unroll 1
-    for (int i = tid; i < F.n; i += kCyThreads) {
+    for (int i = tid; i < F.n; i += cy_nt(CL)) {
         sm[F.f + i] = f[g0 + i];
         if (vin) sm[F.v + i] = vin[g0 + i];
     }
@@ -451,36 +457,55 @@ __global__ void __launch_bounds__(kCyThreads) cycle_cluster_kernel(const __grid_
             break;
         }
         if (l == last && S[l].P == 0 && cap <= 32) {
-            if (tid < 32) cy_warp_sweeps<D2>(l, sm + v, w, citers);
+            if (tid < 32) cy_warp_sweeps<D2, CL>(l, sm + v, w, citers);
             __syncthreads();
             break;
         }
-        cy_smooth<D2>(l, v, t, l < last ? nu1 : citers, w, !(l == first && vin), rank);
+        cy_smooth<D2, CL>(l, v, t, l < last ? nu1 : citers, w, !(l == first && vin), rank);
         if (v != S[l].v) flip |= 1u << l;
         if (l < last) {
-            cy_pass<D2>(l, v, t, w, CY_RESID, rank);
-            cy_sums<D2>(l, t);
+            cy_pass<D2, CL>(l, v, t, w, CY_RESID, rank);
+            cy_sums<D2, CL>(l, t);
         }
     }
 #pragma unroll 1
     for (int l = last - 1; l >= first; --l) {
         const bool in_t = (flip >> l) & 1;
         int v = in_t ? S[l].t : S[l].v, t = in_t ? S[l].v : S[l].t;
-        cy_prolong<D2>(l, v, (flip >> (l + 1)) & 1 ? S[l + 1].t : S[l + 1].v, prolong, rank);
-        cy_smooth<D2>(l, v, t, nu2, w, false, rank);
+        cy_prolong<D2, CL>(l, v, (flip >> (l + 1)) & 1 ? S[l + 1].t : S[l + 1].v, prolong, rank);
+        cy_smooth<D2, CL>(l, v, t, nu2, w, false, rank);
         flip = v == S[l].t ? flip | 1u << l : flip & ~(1u << l);
     }
     // (the last pass ended in a barrier: no CTA leaves while a neighbour reads its planes)
     const float* v = sm + ((flip >> first) & 1 ? F.t : F.v);
     const int n = F.P || rank == 0 ? F.n : 0;  // a replicated first level is written by CTA 0
     if (p64)
-        for (int i = tid; i < n; i += kCyThreads) p64[g0 + i] += (double)v[i];
+        for (int i = tid; i < n; i += cy_nt(CL)) p64[g0 + i] += (double)v[i];
     else
-        for (int i = tid; i < n; i += kCyThreads) vout[g0 + i] = v[i];
+        for (int i = tid; i < n; i += cy_nt(CL)) vout[g0 + i] = v[i];
+}
+
+template <bool D2>
+__global__ void __launch_bounds__(kCyThreads) cycle_cluster_kernel(const __grid_constant__ CyPack C,
+                                                                   const float* __restrict__ image, int first,
+                                                                   const float* f, const float* vin, float* vout,
+                                                                   double* p64, int nu1, int nu2, float w, int citers,
+                                                                   int prolong) {
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    cy_cycle<D2, true>(C, image, (int)rank, first, f, vin, vout, p64, nu1, nu2, w, citers, prolong);
+}
+
+// The cycle of a pack of one CTA from v = 0, as a phase of a 1024-thread persistent kernel
+template <bool D2>
+__device__ __noinline__ void cy_one_cta(const CyPack& C, const float* image, int first, const float* f, float* vout, int nu1,
+                                        int nu2, float w, int citers, int prolong) {
+    cy_cycle<D2, false>(C, image, 0, first, f, nullptr, vout, nullptr, nu1, nu2, w, citers, prolong);
 }
 
 // Layout of a pack of levels (extents e[l] = {nx, ny, nz} of the slab problem) over `ctas` CTAs; false
 // when it does not fit a CTA's shared memory.
+// (dynamic shared bytes of its cycle with and without the stencils: floats, floats - image)
 inline bool cy_layout(CyPack* C, const int (*e)[3], int n, int ctas, bool two_d) {
     if (n < 2 || n > kCyMax) return false;
     C->n = n;
@@ -533,19 +558,18 @@ __device__ __forceinline__ float cy_cell_global(const CyGlobal& G, const float* 
     return cy_cell<D2>(cy_entry(G, i), G.cap, G.ny, G.nxy, f[i], w, mode, v == nullptr,
                        [&](int o) { return v[min(max(i + o, 0), G.n - 1)]; });
 }
+// cell i of a sweep of v (null: from zero) into dst or (p64) added to p64
 template <bool D2>
-__global__ void __launch_bounds__(256) cy_sweep_kernel(float* __restrict__ dst, const float* __restrict__ v,
-                                                       const float* __restrict__ f, CyGlobal G, float w) {
-    wp_pdl_enter();
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i < G.n) dst[i] = cy_cell_global<D2>(G, v, f, i, w, CY_SWEEP);
+__device__ __forceinline__ void cy_sweep_one(float* dst, double* p64, const float* v, const float* f, const CyGlobal& G, float w,
+                                             int i) {
+    const float o = cy_cell_global<D2>(G, v, f, i, w, CY_SWEEP);
+    if (p64) p64[i] += (double)o;
+    else dst[i] = o;
 }
+// coarse cell i of the restricted residual
 template <bool D2>
-__global__ void __launch_bounds__(256) cy_restrict_kernel(float* __restrict__ fc, const float* __restrict__ v,
-                                                          const float* __restrict__ f, CyGlobal G, int cnx, int cny, int cn) {
-    wp_pdl_enter();
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= cn) return;
+__device__ __forceinline__ void cy_restrict_one(float* fc, const float* v, const float* f, const CyGlobal& G, int cnx, int cny,
+                                                int i) {
     const int cz = i / (cnx * cny), rem = i - cz * cnx * cny, x = D2 ? 0 : 2 * (rem / cny), y = 2 * (rem % cny);
     float s = 0.f;
     // cy_sums' order
@@ -561,12 +585,31 @@ __global__ void __launch_bounds__(256) cy_restrict_kernel(float* __restrict__ fc
     }
     fc[i] = s;
 }
+// cell i of v += P vc
+template <bool D2>
+__device__ __forceinline__ void cy_prolong_one(float* v, const float* vc, const CyGlobal& G, int cnx, int cny, int cnz, int kind,
+                                               int i) {
+    const int z = i / G.nxy, rem = i - z * G.nxy, x = D2 ? 0 : rem / G.ny, y = rem - x * G.ny;
+    v[i] += cy_interp<D2>(vc, x, y, z, cnx, cny, cnz, kind);
+}
+template <bool D2>
+__global__ void __launch_bounds__(256) cy_sweep_kernel(float* __restrict__ dst, const float* __restrict__ v,
+                                                       const float* __restrict__ f, CyGlobal G, float w) {
+    wp_pdl_enter();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < G.n) cy_sweep_one<D2>(dst, nullptr, v, f, G, w, i);
+}
+template <bool D2>
+__global__ void __launch_bounds__(256) cy_restrict_kernel(float* __restrict__ fc, const float* __restrict__ v,
+                                                          const float* __restrict__ f, CyGlobal G, int cnx, int cny, int cn) {
+    wp_pdl_enter();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < cn) cy_restrict_one<D2>(fc, v, f, G, cnx, cny, i);
+}
 template <bool D2>
 __global__ void __launch_bounds__(256) cy_prolong_kernel(float* __restrict__ v, const float* __restrict__ vc, CyGlobal G,
                                                          int cnx, int cny, int cnz, int kind) {
     wp_pdl_enter();
     const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= G.n) return;
-    const int z = i / G.nxy, rem = i - z * G.nxy, x = D2 ? 0 : rem / G.ny, y = rem - x * G.ny;
-    v[i] += cy_interp<D2>(vc, x, y, z, cnx, cny, cnz, kind);
+    if (i < G.n) cy_prolong_one<D2>(v, vc, G, cnx, cny, cnz, kind, i);
 }
