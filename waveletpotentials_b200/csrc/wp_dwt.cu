@@ -23,6 +23,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 namespace {
@@ -754,6 +755,13 @@ struct LineJobs {
 };
 constexpr int kLineCP = 33;
 
+// How a CTA's 32 lines are moved.  Strided: a warp takes a position of the lines.  Along y: a warp takes a line,
+// lanes along it; or, where lines of fewer than kLineRun samples leave the CTA few warps, the threads take the
+// samples of the one run of memory that the lines are (1600 lines of 16 samples 11.7 -> 3.7 us, of 64 7.7 -> 5.2;
+// 16384 lines of 128 take 9.4 a line at a time and 11.1 as a run).
+enum { LM_STRIDED = 0, LM_LINES = 1, LM_RUN = 2 };
+constexpr int kLineRun = 128;
+
 __device__ __forceinline__ void cp_async_sample(float* d, const float* s) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(s) : "memory");
 }
@@ -986,7 +994,7 @@ __device__ __forceinline__ void line_run(T* X, T* g, long ps, const LineJob& J, 
     }
 }
 
-template <typename T, bool FWD, bool CONTIG, int P0, int MAXT, int MINB>
+template <typename T, bool FWD, int MOVE, int P0, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) dwt_line_kernel(const __grid_constant__ LineJobs jobs) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     wp_pdl_enter();
@@ -999,8 +1007,21 @@ __global__ void __launch_bounds__(MAXT, MINB) dwt_line_kernel(const __grid_const
     T* dst = static_cast<T*>(J.dst);
     T* X = sm + lane;
     T* g = nullptr;
-    if (CONTIG) {
-        // a warp per line, lanes along it
+    // visits this thread's samples of the run as (offset in the tile, offset in the run)
+    auto run = [&](auto&& fn) {
+        const int nt = blockDim.x, n = min(32, J.lines - l0) * N, dc = nt / N, dp = nt - dc * N;
+        int c = threadIdx.x / N, p = threadIdx.x - c * N;
+        for (int e = threadIdx.x; e < n; e += nt) {
+            fn(p * kLineCP + c, e);
+            p += dp;
+            c += dc;
+            if (p >= N) { p -= N; ++c; }
+        }
+    };
+    if (MOVE == LM_RUN) {
+        const T* from = src + (long)l0 * J.s_in;
+        run([&](int at, int e) { cp_async_sample(sm + at, from + e); });
+    } else if (MOVE == LM_LINES) {
         for (int c = warp; c < 32 && l0 + c < J.lines; c += nw) {
             const T* line = src + (long)(l0 + c) * J.s_in;
             for (int p = lane; p < N; p += 32) cp_async_sample(sm + p * kLineCP + c, line + p);
@@ -1014,9 +1035,12 @@ __global__ void __launch_bounds__(MAXT, MINB) dwt_line_kernel(const __grid_const
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (J.c4) line_run<T, true, FWD, !CONTIG, P0>(X, g, J.pstride, J, warp, lane);
-    else line_run<T, false, FWD, !CONTIG, P0>(X, g, J.pstride, J, warp, lane);
-    if (CONTIG) {
+    if (J.c4) line_run<T, true, FWD, MOVE == LM_STRIDED, P0>(X, g, J.pstride, J, warp, lane);
+    else line_run<T, false, FWD, MOVE == LM_STRIDED, P0>(X, g, J.pstride, J, warp, lane);
+    if (MOVE == LM_RUN) {
+        T* to = dst + (long)l0 * J.s_in;
+        run([&](int at, int e) { to[e] = sm[at]; });
+    } else if (MOVE == LM_LINES) {
         for (int c = warp; c < 32 && l0 + c < J.lines; c += nw) {
             T* line = dst + (long)(l0 + c) * J.s_in;
             for (int p = lane; p < N; p += 32) line[p] = sm[p * kLineCP + c];
@@ -1135,9 +1159,9 @@ bool line_ok(int wavelet, int N) {
     return N - ext <= (sizeof(T) == 4 ? 512 : 256) && (ext ? wavelet == WP_ID_CDF4_6 : wavelet == WP_ID_CDF3_7);
 }
 
-template <typename T, bool FWD, bool CONTIG, int P0, int MAXT, int MINB>
+template <typename T, bool FWD, int MOVE, int P0, int MAXT, int MINB>
 cudaError_t launch_line_k(const LineJobs& jobs, dim3 grid, int nt, size_t smem, cudaStream_t s) {
-    auto kern = dwt_line_kernel<T, FWD, CONTIG, P0, MAXT, MINB>;
+    auto kern = dwt_line_kernel<T, FWD, MOVE, P0, MAXT, MINB>;
     cudaError_t e = wp_set_smem(kern, smem);
     if (e != cudaSuccess) return e;
     wp_launch_pdl(kern, grid, nt, smem, s, jobs);
@@ -1159,24 +1183,21 @@ cudaError_t launch_lines(const LineJobs& jobs, int n, bool contig, bool fwd, cud
     const dim3 grid(wp_cdiv(lines, 32), n);
     const size_t smem = sizeof(T) * (size_t)N * kLineCP;
     const int tok = wp_prof_start(s);
+    // the direction and the way the lines move, for a kernel of at most MAXT threads
+    auto go = [&](auto maxt, auto minb) {
+        constexpr int MAXT = decltype(maxt)::value, MINB = decltype(minb)::value;
+        auto dir = [&](auto move) {
+            constexpr int MOVE = decltype(move)::value;
+            return fwd ? launch_line_k<T, true, MOVE, P0, MAXT, MINB>(jobs, grid, nt, smem, s)
+                       : launch_line_k<T, false, MOVE, P0, MAXT, MINB>(jobs, grid, nt, smem, s);
+        };
+        if (!contig) return dir(std::integral_constant<int, LM_STRIDED>());
+        if (N < kLineRun) return dir(std::integral_constant<int, LM_RUN>());
+        return dir(std::integral_constant<int, LM_LINES>());
+    };
     cudaError_t e;
-    if constexpr (sizeof(T) == 4) {
-        if (nt <= 256)
-            e = fwd ? (contig ? launch_line_k<T, true, true, P0, 256, 3>(jobs, grid, nt, smem, s)
-                              : launch_line_k<T, true, false, P0, 256, 3>(jobs, grid, nt, smem, s))
-                    : (contig ? launch_line_k<T, false, true, P0, 256, 3>(jobs, grid, nt, smem, s)
-                              : launch_line_k<T, false, false, P0, 256, 3>(jobs, grid, nt, smem, s));
-        else
-            e = fwd ? (contig ? launch_line_k<T, true, true, P0, 512, 1>(jobs, grid, nt, smem, s)
-                              : launch_line_k<T, true, false, P0, 512, 1>(jobs, grid, nt, smem, s))
-                    : (contig ? launch_line_k<T, false, true, P0, 512, 1>(jobs, grid, nt, smem, s)
-                              : launch_line_k<T, false, false, P0, 512, 1>(jobs, grid, nt, smem, s));
-    } else {
-        e = fwd ? (contig ? launch_line_k<T, true, true, P0, 512, 1>(jobs, grid, nt, smem, s)
-                          : launch_line_k<T, true, false, P0, 512, 1>(jobs, grid, nt, smem, s))
-                : (contig ? launch_line_k<T, false, true, P0, 512, 1>(jobs, grid, nt, smem, s)
-                          : launch_line_k<T, false, false, P0, 512, 1>(jobs, grid, nt, smem, s));
-    }
+    if (sizeof(T) == 4 && nt <= 256) e = go(std::integral_constant<int, 256>(), std::integral_constant<int, 3>());
+    else e = go(std::integral_constant<int, 512>(), std::integral_constant<int, 1>());
     wp_prof_stop(tok, fwd ? "dwt_forward" : "dwt_inverse", bytes, s);
     return e;
 }
