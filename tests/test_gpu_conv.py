@@ -94,10 +94,12 @@ def test_conv3_rejects_bad_channels(wp):
 
 
 @pytest.mark.parametrize("n,cins,cout", [((201, 16, 16), (16,), 16), ((302, 4, 64), (32,), 32), ((331, 8, 32), (16, 64), 16),
-                                         ((5, 128, 128), (16,), 16), ((1, 4, 4), (32, 16), 64), ((3, 1, 2), (16,), 32)])
+                                         ((5, 128, 128), (16,), 16), ((1, 4, 4), (32, 16), 64), ((3, 1, 2), (16,), 32),
+                                         ((2, 128, 128), (32,), 16), ((3, 128, 128), (32,), 16), ((1, 256, 256), (16,), 16),
+                                         ((7, 256, 256), (16,), 16)])
 def test_conv3_forward_columns_of_planes(wp, oracle, n, cins, cout):
     """Columns of several planes per CTA with a shorter last one, tiles cut by the plane's end, weights of two
-    parts.  Bound: BF16 outputs, as above."""
+    parts; both sides of the rule that leaves few wide planes to the other kernel.  Bound: BF16 outputs, as above."""
     rng = np.random.default_rng(sum(n) + cout)
     xs = [oracle.bf16_round(rng.standard_normal(n + (c,))) for c in cins]
     ws = [oracle.bf16_round(rng.standard_normal((27, cout, c)) / np.sqrt(27 * c)) for c in cins]

@@ -581,8 +581,15 @@ TileGeo tile_geo(int nx, int ny) {
     return g;
 }
 
-// The walk kernel's geometry for a layer, or stages = 0 where the weights and four input planes do not fit
-// shared memory (64 channels on both sides, 96 into 32: those stay with conv3_fwd_kernel).
+// The walk kernel's geometry for a layer, or stages = 0 where conv3_fwd_kernel takes it: where the weights and four
+// input planes do not fit shared memory (64 channels on both sides, 96 into 32), and where few planes make
+// a CTA's start dearer than the input it saves.  Both times in us as fitted to measured ones (B200; within 20%):
+// conv3_fwd_kernel runs waves of two CTAs per SM, 8.6 a part and 0.05 a channel each; the walk kernel pays for the
+// arrival of its first planes (some of it hidden in the waves after the first), then for every plane, 16 channels
+// and CTA on the SM 1.5 of products or, for wide blocks, what they take to arrive.  conv3_fwd_kernel is taken where
+// it is ahead by 2 us.  On planes of 256 x 256, 16 channels: 2 planes 41 against 51 us, 4 planes 69 against 74, 6
+// planes 100 against 92; on 128 x 128, 32 channels: 2 planes 17.6 against 19.3, 3 planes 26.7 against 22.5; one plane
+// of 128 x 128, 16 channels: 15.6 against 13.1.
 WalkGeo walk_geo(int nx, int ny, int nz, int cin0, int cin1, int cout) {
     WalkGeo g{};
     g.pitch = ny + 2;
@@ -608,9 +615,17 @@ WalkGeo walk_geo(int nx, int ny, int nz, int cin0, int cin1, int cout) {
         }
     }
     if (!g.stages) return g;
-    // one wave of CTAs
-    const long slots = (long)ctas * wp_sm_count();
-    g.zc = (int)(((long)g.tiles * nz + slots - 1) / slots);
+    // as many chunks of planes as one wave of CTAs holds, one where it holds no tile of every column
+    const long sms = wp_sm_count(), slots = ctas * sms, chunks = std::max(1L, std::min<long>(nz, slots / g.tiles));
+    g.zc = (int)((nz + chunks - 1) / chunks);
+    const long n = (long)g.tiles * ((nz + g.zc - 1) / g.zc), waves = (n + slots - 1) / slots;
+    const double cin = cin0 + cin1, positions = (double)g.rows * g.pitch;
+    const double start = 5.5 + positions * (0.0032 + 0.00016 * cin), plane = std::max(1.5, 0.0024 * positions) * cin / 16;
+    const double walk = 3.0 + start * (0.4 + 0.6 * waves) + waves * g.zc * plane * std::min<long>(ctas, (n + sms - 1) / sms);
+    const TileGeo t = tile_geo(nx, ny);
+    const long nf = (long)t.nty * t.ntx * nz;
+    const double fwd = 5.0 + (nf + 2 * sms - 1) / (2 * sms) * (8.6 * (cin1 ? 2 : 1) + 0.05 * cin);
+    if (walk > fwd + 2.0) g.stages = 0;
     return g;
 }
 
