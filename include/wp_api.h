@@ -254,8 +254,10 @@ CUWHHD_API wp_status wp_mgfrac3d_tiles(const wp_mgfrac3d* h, int* zc, int* varia
    (level and zc ignored): the levels below the finest run as one persistent cooperative launch
    (variant 1, where the autotuner finds it faster) or launch by launch (variant 0, the default).
    The small levels (cubes from 32^3, 2D grids from 256^2) otherwise run as one launch of one
-   thread-block cluster; a level pinned with kind 0 or 1 (or 4: level 0) and every level above it
-   keep kernels of their own. */
+   thread-block cluster; a level pinned with kind 0 or 1 and every level above it run kernels of
+   their own, until a call with zc < 0 takes the pin away.  Kind 4 (level ignored): level 0's V(2,2)
+   cycle as two fused kernels (variant 1, zc planes per CTA) or kernel by kernel (variant 0), level 0
+   pinned likewise. */
 CUWHHD_API wp_status wp_mgfrac3d_set_tile(wp_mgfrac3d* h, int level, int kind, int zc, int variant);
 /* Uniform rows of one level (no reference counterpart): the number of (x, z) rows of cells whose
    interior face fractions are all exactly 1, which the column kernels stream without reading any

@@ -74,13 +74,31 @@ def test_cluster_cycles_match_oracle(wp, oracle, n, nu1, nu2, prolong):
 
 
 def test_pinned_level_keeps_its_own_kernels(wp, oracle):
-    """A level pinned with SetTile is not part of the single launch; the cycles stay the same."""
+    """A level pinned with SetTile is not part of the single launch, until it is given back; the cycles stay the same."""
     n = (32, 32, 32)
     h, a, act, f = _problem(oracle, n, seed=3)
     ref = oracle.mgfrac3d_solve(f, *a, n, (h,) * 3, 3, 2, 2, 2 / 3, prolong=1)[0]
-    for pinned in (0, 1, 2):
-        mg = wp.CuMultigridFrac3D(*[T(v) for v in a], n, h)
-        mg.SetTile(pinned, 0, 0, 0)
+    mg = wp.CuMultigridFrac3D(*[T(v) for v in a], n, h)
+    tf = T(f)
+
+    def solve():
         out = torch.zeros(f.shape, device="cuda")
-        mg.SolveTol(out, None, T(f), rel_tol=0.0, max_cycles=3, precision=wp.PREC_FP32)
+        c0 = wp.lib().wp_launch_count()
+        mg.SolveTol(out, None, tf, rel_tol=0.0, max_cycles=3, precision=wp.PREC_FP32)
         _close(ref, out.double().cpu().numpy(), act, 1.2e-5)
+        return out, wp.lib().wp_launch_count() - c0
+
+    whole, launches = solve()
+    for pin, back in (((0, 0, 0, 0), (0, 0, -1, 0)), ((1, 0, 4, 0), (1, 0, -1, 0)), ((2, 1, 0, 1), (2, 1, -1, 0)),
+                      ((0, 4, 0, 0), (0, 4, -1, 1)), ((0, 4, 8, 1), (0, 4, -1, 1))):
+        mg.SetTile(*pin)
+        assert solve()[1] > launches, pin
+        mg.SetTile(*back)
+        out, again = solve()
+        assert again == launches and torch.equal(out, whole), back
+    mg.SetTile(1, 0, 4, 0)  # every pin counts
+    mg.SetTile(2, 1, 4, 0)
+    for back in ((2, 1, -1, 0), (1, 0, -1, 0)):
+        assert solve()[1] > launches
+        mg.SetTile(*back)
+    assert solve()[1] == launches

@@ -1,5 +1,5 @@
-"""Prolongation by pairs of planes (quads) and by four planes (any extents): one V(0, 1) cycle's correction of levels
-with odd and even numbers of planes, against the FP64 oracle."""
+"""Prolongation by pairs of planes (quads) and by four planes (any extents): V(1, 1) cycles of levels with odd and even
+numbers of planes, against the FP64 oracle."""
 import pytest
 import torch
 

@@ -2234,6 +2234,7 @@ struct Level {
                       // 3 = two sweeps per launch, 4 = TMA-staged rows, 5 = cp.async-pipelined planes,
                       // 6 = one cell per thread; restrict: 0-2 register budgets, 3 = pipelined,
                       // 4 = one cell per thread; defect: 0 quads, 1 pipelined)
+    unsigned pinned;  // bit k: kind k (kZcJacobi, kZcRestrict) pinned by wp_mgfrac3d_set_tile
     int* err;         // the handle's device error flag (bounded waits of the TMA-staged kernel)
     // index-sparse cycle (built by the first wp_mgfrac3d_solve_index)
     unsigned* imask;  // per 32-cell segment of a row: the selected cells
@@ -2550,6 +2551,7 @@ struct wp_mgfrac3d {
     long long loop_launches[2]; // kernels of the first cycle's graph part and of one loop body
     CyPlan cy;         // the small levels' single-launch cycle (FP32): its levels are cy.l0 .. nl - 1
     int cy_from;       // levels above this one run their own kernels (wp_mgfrac3d_set_tile pins a level)
+    int fz_pinned;     // level 0's cycle is pinned to its fused kernels or to their counterparts
     CyPlan one;        // the levels of the pack that one CTA holds (see one_cta_plan)
     int shares;        // the handle shares the device (see wp_mg_share_device)
     int fz_on;         // run the V(2,2) FP32 cycle of level 0 as the two fused kernels where it fits
@@ -5021,8 +5023,15 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_tiles(const wp_mgfrac3d* h, int* zc,
     return WP_OK;
 }
 
+// A pinned level and every level above it run their own kernels.
+static void set_cy_from(wp_mgfrac3d* h) {
+    h->cy_from = h->fz_pinned ? 1 : 0;
+    for (int l = 0; l < h->nl; ++l)
+        if (h->lv[l].pinned) h->cy_from = l + 1;
+}
+
 // Pins the chunk and kernel variant of one level's column kernel (kind 0 jacobi, 1 restrict,
-// 2 defect); zc <= 0 restores the heuristic.
+// 2 defect); zc <= 0 restores the heuristic, zc < 0 also takes the pin away.
 extern "C" CUWHHD_API wp_status wp_mgfrac3d_set_tile(wp_mgfrac3d* h, int level, int kind, int zc, int variant) {
     if (h && kind == 3 && (variant == 0 || variant == 1)) {
         // the levels below the finest: one persistent launch (1) or launch by launch (0)
@@ -5038,7 +5047,8 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_set_tile(wp_mgfrac3d* h, int level, 
         // level 0's V(2,2) cycle: the two fused kernels (1) or one kernel per sweep / transfer (0)
         h->fz_on = variant;
         h->fz_zc = zc > 0 ? zc + (zc & 1) : 0;
-        h->cy_from = std::max(h->cy_from, 1);  // a pinned level runs its own kernels
+        h->fz_pinned = zc >= 0;
+        set_cy_from(h);
         ++h->tune_gen;
         return WP_OK;
     }
@@ -5051,7 +5061,11 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_set_tile(wp_mgfrac3d* h, int level, 
     L.zc[kind] = zc > 0 ? zc : 0;
     L.var[kind] = variant;
     L.zc_ms[kind] = 0.f;
-    if (kind != kZcDefect) h->cy_from = std::max(h->cy_from, level + 1);  // a pinned level runs its own kernels
+    if (kind != kZcDefect) {
+        const unsigned bit = 1u << kind;
+        L.pinned = zc >= 0 ? L.pinned | bit : L.pinned & ~bit;
+        set_cy_from(h);
+    }
     ++h->tune_gen;
     return WP_OK;
 }
