@@ -77,6 +77,12 @@ CUWHHD_API int wp_version(void);
 #define WP_WAIT_SITE_BATCH_PUBLISH 3
 CUWHHD_API wp_status wp_debug_withhold_wait(int site, int at, double limit_seconds);
 
+/* Gives the device memory that the library keeps between calls back to the driver, on every device (no
+   reference counterpart).  Kept is at most 64 MB per device, scratch of the level-set calls
+   (wp_fractions3d_subsampled, wp_fast_sweep_*, wp_particles_to_ls*), which have no handle; blocks whose
+   call has not finished on its stream stay.  Destroying any handle does the same. */
+CUWHHD_API wp_status wp_release_scratch(void);
+
 /* Instrumentation (no reference counterpart): number of kernels this library has launched since
    the last reset, and optional per-kernel-class timing with CUDA events on the launching stream.
    wp_profile_collect() synchronizes the device and returns the number of kernel classes;

@@ -105,3 +105,29 @@ def test_particles_to_ls_narrow_matches_reference_and_oracle(wp, oracle, start):
     torch.cuda.synchronize()
     assert np.abs(N(ls) - ref).max() <= 1e-5 * np.abs(ref).max()
     assert float(buf[:4096].min()) == 12345.0 and float(buf[4096 + cells:].min()) == 12345.0
+
+
+def test_kept_scratch_is_given_back(wp):
+    """The scratch that the calls keep (here 32 MB) stays below its bound and goes back to the driver on request and with
+    a handle of any kind."""
+    n = (256, 256, 128)
+    ls = torch.rand((n[2], n[0], n[1]), device="cuda") - 0.5
+    free = lambda: (torch.cuda.synchronize(), torch.cuda.mem_get_info()[0])[1]  # noqa: E731
+    wp.release_scratch()
+    before = free()
+
+    def keep():
+        wp.CuFastSweeping.Solve(ls, n, 1.0 / 256, 1)
+        kept = before - free()
+        assert (32 << 20) <= kept <= (64 << 20) + (4 << 20), kept
+
+    keep()
+    wp.release_scratch()
+    assert free() == before
+    for handle in (lambda: wp.CuDst3D((8, 8, 8), (0.1,) * 3), lambda: wp.CuWaveletPotentialRecover2D((8, 8), (0.1,) * 2, "n")):
+        h = handle()
+        keep_less = before - free()
+        wp.CuFastSweeping.Solve(ls, n, 1.0 / 256, 1)
+        assert before - free() >= keep_less + (32 << 20)
+        h.close()
+        assert before - free() <= keep_less

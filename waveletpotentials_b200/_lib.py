@@ -55,6 +55,7 @@ SIGNATURES = {
     "wp_last_error": (ctypes.c_char_p, []),
     "wp_version": (I, []),
     "wp_debug_withhold_wait": (I, [I, I, ctypes.c_double]),
+    "wp_release_scratch": (I, []),
     "wp_profile_enable": (None, [I]),
     "wp_profile_reset": (None, []),
     "wp_launch_count": (ctypes.c_longlong, []),

@@ -942,6 +942,12 @@ class BatchProjector:
 
 
 # ------------------------------------------------------------------ test-only failure injection
+def release_scratch():
+    """Gives the device memory that the level-set calls keep between them (at most 64 MB per device) back
+    to the driver (wp_release_scratch)."""
+    check(lib().wp_release_scratch(), "wp_release_scratch")
+
+
 def debug_withhold_wait(site, at=0, limit_s=1e-3):
     """Test only: the next launch at ``site`` (``WAIT_SITE_GRID_BARRIER``: the persistent
     below-finest multigrid cycle; ``WAIT_SITE_CONV_PIPELINE``: the tensor-core convolutions) leaves

@@ -659,6 +659,7 @@ extern "C" CUWHHD_API wp_status wp_batch_destroy(wp_batch* B) {
     if (B->d_slots) cudaFree((void*)B->d_slots);
     if (B->d_loops) cudaFree((void*)B->d_loops);
     if (B->d_out) cudaFree(B->d_out);
+    wp_scratch_trim();
     delete B;
     return WP_OK;
 }

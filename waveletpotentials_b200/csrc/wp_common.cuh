@@ -58,8 +58,9 @@ cudaError_t wp_read_small(void* host, const void* dev, size_t bytes, cudaStream_
 bool wp_profile_is_enabled();
 // Stream-ordered device scratch from the library's own bounded pool; freed with cudaFreeAsync.
 cudaError_t wp_scratch_alloc(void** p, size_t bytes, cudaStream_t s);
-// gives the current device's unused scratch back
-void wp_scratch_trim();
+// gives the unused scratch of every device back (called where a handle is destroyed, after its frees, which wait
+// for the scratch in use)
+cudaError_t wp_scratch_trim();
 template <typename T>
 wp_status wp_dwt_axis_tune(T* buf, int DX, int DY, int DZ, int levels, char axis, int wavelet, char bc, int forward,
                            cudaStream_t s);

@@ -299,6 +299,7 @@ extern "C" CUWHHD_API wp_status wp_dst3d_solve(wp_dst3d* h, double* dst, const d
 extern "C" CUWHHD_API wp_status wp_dst3d_destroy(wp_dst3d* h) {
     if (!h) return WP_OK;
     for (int a = 0; a < 3; ++a) if (h->M[a]) cudaFree(h->M[a]);
+    wp_scratch_trim();
     delete h;
     return WP_OK;
 }

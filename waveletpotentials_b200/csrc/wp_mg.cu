@@ -4736,11 +4736,11 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_iterate64_view(wp_mgfrac3d* h, const
 
 extern "C" CUWHHD_API wp_status wp_mgfrac3d_destroy(wp_mgfrac3d* h) {
     if (!h) return WP_OK;
-    wp_scratch_trim();
     destroy_loop_graph(h);
     if (h->loop_state) cudaFree(h->loop_state);
     if (h->loop_cap) cudaStreamDestroy(h->loop_cap);
     destroy_levels(h);
+    wp_scratch_trim();
     delete h;
     return WP_OK;
 }

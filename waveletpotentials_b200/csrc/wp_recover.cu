@@ -460,11 +460,11 @@ extern "C" CUWHHD_API wp_status wp_recover3d_create(wp_recover3d** out, int nx, 
 
 extern "C" CUWHHD_API wp_status wp_recover3d_destroy(wp_recover3d* h) {
     if (!h) return WP_OK;
-    wp_scratch_trim();
     for (int a = 0; a < 3; ++a) {
         if (h->tab[a]) cudaFree(h->tab[a]);
         if (h->tmp[a]) cudaFree(h->tmp[a]);
     }
+    wp_scratch_trim();
     delete h;
     return WP_OK;
 }
@@ -679,6 +679,7 @@ extern "C" CUWHHD_API wp_status wp_recover2d_destroy(wp_recover2d* h) {
         if (h->tab[a]) cudaFree(h->tab[a]);
         if (h->tmp[a]) cudaFree(h->tmp[a]);
     }
+    wp_scratch_trim();
     delete h;
     return WP_OK;
 }

@@ -277,6 +277,7 @@ extern "C" CUWHHD_API wp_status wp_sweep3d_destroy(wp_sweep3d* h) {
     if (!h) return WP_OK;
     if (h->dst) wp_dst3d_destroy(h->dst);
     if (h->phi) cudaFree(h->phi);
+    wp_scratch_trim();
     delete h;
     return WP_OK;
 }

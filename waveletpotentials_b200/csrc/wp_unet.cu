@@ -664,6 +664,7 @@ extern "C" CUWHHD_API wp_status wp_unet_destroy(wp_unet* h) {
     if (!h) return WP_OK;
     cudaDeviceSynchronize();
     for (void* p : h->allocs) cudaFree(p);
+    wp_scratch_trim();
     delete h;
     return WP_OK;
 }

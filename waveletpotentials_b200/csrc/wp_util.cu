@@ -30,8 +30,9 @@ int wp_sm_count() {
 // Stream-ordered scratch from a memory pool of the library's own, one per device, that keeps up to
 // kScratchKeep bytes between calls (the default pool returns everything to the driver at the next
 // synchronisation, and the next allocation then costs about a millisecond).  What is above that goes back as
-// before, the rest when a solver or transform handle is destroyed (wp_scratch_trim); freed with cudaFreeAsync.  Thread- and stream-safe as the runtime's pools are.  A
-// stream that is being captured keeps the default pool (the allocation becomes a node of the graph).
+// before; the rest, on every device, with wp_release_scratch and whenever a handle of any kind is destroyed.
+// Freed with cudaFreeAsync; thread- and stream-safe as the runtime's pools are.  A stream that is being captured
+// keeps the default pool (the allocation becomes a node of the graph).
 #include <mutex>
 
 namespace {
@@ -68,12 +69,20 @@ cudaError_t wp_scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
     return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
-// gives the current device's unused scratch back to the driver
-void wp_scratch_trim() {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+// gives the unused scratch of every device back to the driver
+cudaError_t wp_scratch_trim() {
     std::lock_guard<std::mutex> lk(g_scratch_mu);
-    if (g_scratch_pool[dev]) cudaMemPoolTrimTo(g_scratch_pool[dev], 0);
+    cudaError_t r = cudaSuccess;
+    for (cudaMemPool_t pool : g_scratch_pool) {
+        const cudaError_t e = pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
+        if (r == cudaSuccess) r = e;
+    }
+    return r;
+}
+
+extern "C" CUWHHD_API wp_status wp_release_scratch(void) {
+    WP_CUDA_TRY(wp_scratch_trim());
+    return WP_OK;
 }
 
 extern "C" CUWHHD_API const char* wp_last_error(void) { return g_err; }
