@@ -77,6 +77,10 @@ CUWHHD_API int wp_version(void);
 #define WP_WAIT_SITE_BATCH_PUBLISH 3
 CUWHHD_API wp_status wp_debug_withhold_wait(int site, int at, double limit_seconds);
 
+/* Test-only: the next multigrid handle is created as on a device that places thread-block clusters of at
+   most `ctas` CTAs (0: none; < 0: as the device is).  One shot.  No reference counterpart. */
+CUWHHD_API wp_status wp_debug_cluster_limit(int ctas);
+
 /* Gives the device memory that the library keeps between calls back to the driver, on every device (no
    reference counterpart).  Kept is at most 64 MB per device, scratch of the level-set calls
    (wp_fractions3d_subsampled, wp_fast_sweep_*, wp_particles_to_ls*), which have no handle; blocks whose

@@ -102,3 +102,31 @@ def test_pinned_level_keeps_its_own_kernels(wp, oracle):
         assert solve()[1] > launches
         mg.SetTile(*back)
     assert solve()[1] == launches
+
+
+@pytest.mark.parametrize("ctas", [8, 4, 2, 1, 0])
+@pytest.mark.parametrize("n", [(32, 32, 32), (33, 17, 9), (7, 3, 65), (256, 256)])
+def test_smaller_clusters_match_oracle(wp, oracle, n, ctas):
+    """A device that places smaller clusters only, or none: fewer levels in the launch, the same cycles.  Bound as above,
+    or that of a finest level with kernels of its own: they round f - sum(c v) by eps v / h^2, white noise whose smoothest
+    mode (1 / N of it) the cycle divides by an eigenvalue 8 N^2 / pi^2 below the coefficients: 0.8 N eps32, twice that
+    for its neighbours."""
+    bound = max(1.2e-5, 1.6 * max(n) * 6e-8)
+    h, a, act, f = _problem(oracle, n, seed=sum(n) + ctas)
+    solve = oracle.mgfrac3d_solve if len(n) == 3 else oracle.mgfrac2d_solve
+    ref = solve(f, *a, n, (h,) * len(n), 4, 2, 2, 2 / 3, prolong=1)[0]
+    results = []
+    for limit in (ctas, -1):
+        wp.debug_cluster_limit(limit)
+        mg = (wp.CuMultigridFrac3D if len(n) == 3 else wp.CuMultigridFrac2D)(*[T(v) for v in a], n, h)
+        out = torch.full(f.shape, float("nan"), device="cuda")
+        c0 = wp.lib().wp_launch_count()
+        rep = mg.SolveTol(out, None, T(f), rel_tol=0.0, max_cycles=4, precision=wp.PREC_FP32)
+        results.append((out, wp.lib().wp_launch_count() - c0))
+        assert rep["status"] == "WP_OK" and rep["cycles"] == 4
+        _close(ref, out.double().cpu().numpy(), act, bound)
+    (less, launches), (whole, launches16) = results
+    if ctas >= 4 and n == (33, 17, 9) or ctas and n == (7, 3, 65):  # still the whole grid: the same bits
+        assert launches == launches16 and torch.equal(less, whole)
+    else:
+        assert launches > launches16

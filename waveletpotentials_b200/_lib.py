@@ -56,6 +56,7 @@ SIGNATURES = {
     "wp_version": (I, []),
     "wp_debug_withhold_wait": (I, [I, I, ctypes.c_double]),
     "wp_release_scratch": (I, []),
+    "wp_debug_cluster_limit": (I, [I]),
     "wp_profile_enable": (None, [I]),
     "wp_profile_reset": (None, []),
     "wp_launch_count": (ctypes.c_longlong, []),

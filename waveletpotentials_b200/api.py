@@ -948,6 +948,12 @@ def release_scratch():
     check(lib().wp_release_scratch(), "wp_release_scratch")
 
 
+def debug_cluster_limit(ctas):
+    """Test-only: the next multigrid handle is created as on a device that places thread-block clusters of
+    at most ``ctas`` CTAs (wp_debug_cluster_limit).  One shot."""
+    check(lib().wp_debug_cluster_limit(int(ctas)), "wp_debug_cluster_limit")
+
+
 def debug_withhold_wait(site, at=0, limit_s=1e-3):
     """Test only: the next launch at ``site`` (``WAIT_SITE_GRID_BARRIER``: the persistent
     below-finest multigrid cycle; ``WAIT_SITE_CONV_PIPELINE``: the tensor-core convolutions) leaves

@@ -19,6 +19,7 @@
 #include "wp_tc.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <map>
 #include <mutex>
@@ -2693,10 +2694,42 @@ cudaError_t cy_prepare() {
     return e;
 }
 
+// Test only (wp_debug_cluster_limit): the largest cluster that the next handle's plan may count on.
+std::atomic<int> g_cluster_limit{-1};
+
+// the launch of a pack's cluster, at[2] its attributes
+cudaLaunchConfig_t cycle_config(const CyPack& pack, cudaLaunchAttribute* at, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pack.ctas);
+    cfg.blockDim = dim3(kCyThreads);
+    cfg.dynamicSmemBytes = sizeof(float) * (size_t)pack.floats;
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = pack.ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = s == nullptr || s == cudaStreamLegacy || s == cudaStreamPerThread ? 1 : 2;
+    return cfg;
+}
+
+// whether the device places the pack's cluster (a GPC may have fewer SMs free than it has, and a context fewer still)
+bool cluster_placed(const CyPack& pack, bool d2, cudaStream_t s) {
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = cycle_config(pack, at, s);
+    int n = 0;
+    const cudaError_t e = d2 ? cudaOccupancyMaxActiveClusters(&n, cycle_cluster_kernel<true>, &cfg)
+                             : cudaOccupancyMaxActiveClusters(&n, cycle_cluster_kernel<false>, &cfg);
+    (void)cudaGetLastError();
+    return e == cudaSuccess && n > 0;
+}
+
 // The pack of small levels: the finest level from which all the rest fits the shared memory of up to `most`
-// CTAs (a cluster of 16 needs the non-portable size; B200 places it on one GPC).  With 16, cubes from 32^3
-// and 2D grids from 256^2; a cycle from there takes 31 and 50 us, where launches took 75 (from 32^3) and 110.
-wp_status build_cycle_plan(wp_mgfrac3d* h, CyPlan* q, int most, cudaStream_t s) {
+// CTAs, or of the largest cluster below that which the device places (16 need the non-portable size; B200 places
+// them on one GPC).  With 16, cubes from 32^3 and 2D grids from 256^2; a cycle from there takes 31 and 50 us,
+// where launches took 75 (from 32^3) and 110.  None: every level runs launch by launch.
+void choose_pack(wp_mgfrac3d* h, CyPlan* q, int most) {
     const bool d2 = h->dims == 2;
     q->l0 = h->nl;
     for (int l = 0; l + 2 <= h->nl; ++l) {
@@ -2714,8 +2747,16 @@ wp_status build_cycle_plan(wp_mgfrac3d* h, CyPlan* q, int most, cudaStream_t s) 
             break;
         }
     }
-    if (q->l0 == h->nl) return WP_OK;
+}
+wp_status build_cycle_plan(wp_mgfrac3d* h, CyPlan* q, int most, cudaStream_t s) {
+    const bool d2 = h->dims == 2;
     WP_CUDA_TRY(d2 ? cy_prepare<true>() : cy_prepare<false>());
+    for (q->l0 = h->nl; most > 0; most /= 2) {
+        choose_pack(h, q, most);
+        if (q->l0 == h->nl || cluster_placed(q->pack, d2, s)) break;
+        q->l0 = h->nl;
+    }
+    if (q->l0 == h->nl) return WP_OK;
     WP_CUDA_TRY(cudaMalloc((void**)&q->image, sizeof(float) * (size_t)q->pack.image * q->pack.ctas));
     WP_CUDA_TRY(cudaMemsetAsync(q->image, 0, sizeof(float) * (size_t)q->pack.image * q->pack.ctas, s));
     for (int k = 0; k < q->pack.n; ++k) {
@@ -2747,19 +2788,8 @@ CyGlobal cy_global(const wp_mgfrac3d* h, int l) {
 // the cycle from level l of the pack (see cycle_cluster_kernel)
 cudaError_t launch_cycle_cluster(const wp_mgfrac3d* h, const CyPlan& q, int l, const float* f, const float* vin, float* vout,
                                  double* p64, int nu1, int nu2, float w, int prolong, cudaStream_t s) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(q.pack.ctas);
-    cfg.blockDim = dim3(kCyThreads);
-    cfg.dynamicSmemBytes = sizeof(float) * (size_t)q.pack.floats;
-    cfg.stream = s;
     cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = q.pack.ctas;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = s == nullptr || s == cudaStreamLegacy || s == cudaStreamPerThread ? 1 : 2;
+    const cudaLaunchConfig_t cfg = cycle_config(q.pack, at, s);
     auto k = h->dims == 2 ? cycle_cluster_kernel<true> : cycle_cluster_kernel<false>;
     return cudaLaunchKernelEx(&cfg, k, q.pack, (const float*)q.image, l - q.l0, f, vin, vout, p64, nu1, nu2, w,
                               h->coarsest_iters, prolong);
@@ -3253,7 +3283,8 @@ wp_status create_common(wp_mgfrac3d** out, int dims, const float* ax, const floa
     h->mid_on = 0;
     h->fz_on = 1;
     wp_status st = build_hierarchy(h, ax, ay, az, nx, ny, nz, dx, dy, dz, s);
-    if (st == WP_OK) st = build_cycle_plan(h, &h->cy, 16, s);
+    const int limit = g_cluster_limit.exchange(-1);
+    if (st == WP_OK) st = build_cycle_plan(h, &h->cy, limit < 0 ? 16 : std::min(limit, 16), s);
     if (st == WP_OK) {
         cudaError_t e = cudaMalloc((void**)&h->acc, 4 * sizeof(double) + 16);
         // the int error flag lives in the 16 bytes after the four FP64 slots
@@ -5067,6 +5098,11 @@ extern "C" CUWHHD_API wp_status wp_mgfrac3d_set_tile(wp_mgfrac3d* h, int level, 
         set_cy_from(h);
     }
     ++h->tune_gen;
+    return WP_OK;
+}
+
+extern "C" CUWHHD_API wp_status wp_debug_cluster_limit(int ctas) {
+    g_cluster_limit = ctas;
     return WP_OK;
 }
 
