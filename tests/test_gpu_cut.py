@@ -61,3 +61,25 @@ def test_cut_matches_oracle_in_place(wp, oracle, n, level):
     with pytest.raises(wp.WPError):
         rec.CutCoefficients(*t, *t, int(np.log2(min(n))) + 1)
     rec.close()
+
+
+@pytest.mark.parametrize("n,level", [((64, 64, 64), 2), ((32, 128, 64), 3), ((1024, 4, 4), 1)])
+def test_cut_into_the_buffers_of_other_inputs(wp, n, level):
+    """Outputs in the storage of the inputs that come before them: the components go in turn."""
+    s = wp.mac_shapes3d(*n)
+    keys = ("qx", "qy", "qz")
+    g = torch.Generator(device="cuda").manual_seed(level)
+    q = [torch.randn(tuple(s[k]), device="cuda", generator=g) for k in keys]
+    rec = wp.CuWaveletPotentialRecover3D(n, 1.0 / n[0])
+    want = [torch.empty_like(t) for t in q]
+    rec.CutCoefficients(*want, *q, level)
+    store = [torch.zeros(max(t.numel() for t in q), device="cuda") for _ in range(4)]
+    view = lambda b, k: store[b][:int(np.prod(s[k]))].view(tuple(s[k]))  # noqa: E731
+    src = [view(b, k) for b, k in enumerate(keys)]
+    dst = [view(b, k) for b, k in zip((3, 0, 1), keys)]
+    for a, b in zip(src, q):
+        a.copy_(b)
+    rec.CutCoefficients(*dst, *src, level)
+    torch.cuda.synchronize()
+    for a, b in zip(dst, want):
+        assert torch.equal(a, b)

@@ -1297,10 +1297,19 @@ wp_status wp_dwt_axis_launch(T* dst, const T* src, int DX, int DY, int DZ, int l
     return WP_OK;
 }
 
-// up to three passes along one axis, in one launch where dwt_line_kernel takes them all
+// up to three passes along one axis, in one launch where dwt_line_kernel takes them all and none writes what another
+// reads (a caller may give one component's input as another's output: then they run in turn)
 wp_status wp_dwt_axis_launch_n(const WpDwtPass* q, int n, int levels, char axis, int forward, cudaStream_t stream) {
     LineJobs jobs{};
     bool one = true;
+    auto apart = [](const float* a, const WpDwtPass& p, const float* b, const WpDwtPass& q) {
+        const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+        const size_t nx = sizeof(float) * (size_t)p.DX * p.DY * p.DZ, ny = sizeof(float) * (size_t)q.DX * q.DY * q.DZ;
+        return x + nx <= y || y + ny <= x;
+    };
+    for (int k = 0; k < n; ++k)
+        for (int j = 0; j < n; ++j)
+            if (j != k) one = one && apart(q[k].dst, q[k], q[j].src, q[j]);
     int contig = 0;
     for (int k = 0; k < n; ++k) {
         TileGeom g;
