@@ -2524,7 +2524,40 @@ bool launch_cycle_up(const Level& L, const Level& C, float* dst, double* p64, co
 
 }  // namespace
 
+// Device memory of a handle, carved from a few allocations.  A driver allocation costs about 0.3 ms, and so does its
+// release; with one per array that was most of a handle's creation (32^3 1.16 -> 0.68 ms, 2D 256^2 1.7 -> 0.8,
+// 201 x 150 x 101 5.6 -> 0.9).
+struct HandleMem {
+    std::vector<void*> chunks;
+    char* at = nullptr;
+    size_t left = 0, chunk = 0;  // chunk: at least what the next allocation takes
+    template <typename T>
+    cudaError_t get(T** p, size_t bytes) {
+        bytes = (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+        if (bytes > left) {
+            void* q = nullptr;
+            const size_t size = std::max(bytes, chunk);
+            const cudaError_t e = cudaMalloc(&q, size);
+            if (e != cudaSuccess) return e;
+            chunks.push_back(q);
+            at = static_cast<char*>(q);
+            left = size;
+            chunk = 0;
+        }
+        *p = reinterpret_cast<T*>(at);
+        at += bytes;
+        left -= bytes;
+        return cudaSuccess;
+    }
+    void free() {
+        for (void* q : chunks) cudaFree(q);
+        chunks.clear();
+        left = 0;
+    }
+};
+
 struct wp_mgfrac3d {
+    HandleMem mem;     // the levels' arrays, the packs' stencils, acc
     int dims;          // 2 or 3 (2D problems use nz = 1)
     int last64;        // 0: none, 1: p64 (mixed), 2: lv[0].v64 (fp64) holds the last FP64 iterate
     int nl;
@@ -2564,23 +2597,46 @@ struct wp_mgfrac3d {
 
 namespace {
 
+void choose_pack(wp_mgfrac3d* h, CyPlan* q, int most);
+
+// The levels' extents (halved, rounded up, while every one is above 1), and the memory that they take with a
+// pack over up to `most` CTAs as the first allocation.
+void size_levels(wp_mgfrac3d* h, const int* ext, int most) {
+    int n[3] = {ext[0], ext[1], ext[2]};
+    const int dims = h->dims;
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    size_t total = up(4 * sizeof(double) + 16);
+    h->nl = 0;
+    while (std::min(n[0], std::min(n[1], dims == 2 ? n[1] : n[2])) > 1 && h->nl < kMaxLevels) {
+        Level& L = h->lv[h->nl++];
+        for (int a = 0; a < 3; ++a) L.n[a] = n[a];
+        L.cells = (long)n[0] * n[1] * n[2];
+        const size_t planes = n[2], rows = n[0], cols = n[1], sum = rows + cols + planes;
+        total += up(4 * (rows + 1) * cols * planes) + up(4 * rows * (cols + 1) * planes) +
+                 up(dims == 2 ? 4 : 4 * rows * cols * (planes + 1)) + 4 * up(4 * (size_t)L.cells) + up(rows * planes) +
+                 up(8 * 3 * sum) + up(4 * (2 * sum + planes));
+        if (dims == 3 && fz_level_ok(n)) total += up((rows / fz::TX) * (cols / fz::TY) * planes);
+        for (int a = 0; a < dims; ++a) n[a] = wp_half_up(n[a]);
+    }
+    CyPlan q;
+    choose_pack(h, &q, most);
+    if (q.l0 < h->nl) total += up(sizeof(float) * (size_t)q.pack.image * q.pack.ctas);
+    h->mem.chunk = total;
+}
+
 wp_status build_hierarchy(wp_mgfrac3d* h, const float* ax, const float* ay, const float* az, int nx, int ny, int nz,
                           double dx, double dy, double dz, cudaStream_t s) {
-    int n[3] = {nx, ny, nz};
     const int dims = h->dims;
-    auto mn = [&](const int* e) { return dims == 2 ? (e[0] < e[1] ? e[0] : e[1]) : std::min(e[0], std::min(e[1], e[2])); };
     std::vector<double> hd[3];
     hd[0].assign(nx, dx);
     hd[1].assign(ny, dy);
     hd[2].assign(nz, dz);
-    int nl = 0;
-    while (mn(n) > 1 && nl < kMaxLevels) {
+    for (int nl = 0; nl < h->nl; ++nl) {
         Level& L = h->lv[nl];
-        for (int a = 0; a < 3; ++a) L.n[a] = n[a];
-        L.cells = (long)n[0] * n[1] * n[2];
+        const int* n = L.n;
         const long fs[3] = {(long)(n[0] + 1) * n[1] * n[2], (long)n[0] * (n[1] + 1) * n[2],
                             dims == 2 ? 1 : (long)n[0] * n[1] * (n[2] + 1)};
-        for (int a = 0; a < 3; ++a) WP_CUDA_TRY(cudaMalloc((void**)&L.frac[a], sizeof(float) * fs[a]));
+        for (int a = 0; a < 3; ++a) WP_CUDA_TRY(h->mem.get(&L.frac[a], sizeof(float) * fs[a]));
         if (nl == 0) {
             WP_CUDA_TRY(cudaMemcpyAsync(L.frac[0], ax, sizeof(float) * fs[0], cudaMemcpyDeviceToDevice, s));
             WP_CUDA_TRY(cudaMemcpyAsync(L.frac[1], ay, sizeof(float) * fs[1], cudaMemcpyDeviceToDevice, s));
@@ -2595,13 +2651,13 @@ wp_status build_hierarchy(wp_mgfrac3d* h, const float* ax, const float* ay, cons
             }
             if (dims == 2) WP_CUDA_TRY(cudaMemsetAsync(L.frac[2], 0, sizeof(float), s));
         }
-        WP_CUDA_TRY(cudaMalloc((void**)&L.fyc, sizeof(float) * L.cells));
+        WP_CUDA_TRY(h->mem.get(&L.fyc, sizeof(float) * L.cells));
         WP_KERNEL("fyc", 8.0 * L.cells, s,
                   fyc_kernel<<<std::min<unsigned>(wp_cdiv(L.cells, 256), 4096), 256, 0, s>>>(L.fyc, L.frac[1], n[0],
                                                                                              n[1], L.cells));
         if (dims == 3 && fz_level_ok(n)) {
             const int ntiles = (n[0] / fz::TX) * (n[1] / fz::TY);
-            WP_CUDA_TRY(cudaMalloc((void**)&L.tuni, (size_t)ntiles * n[2]));
+            WP_CUDA_TRY(h->mem.get(&L.tuni, (size_t)ntiles * n[2]));
             Lvl<float> V{};
             V.nx = n[0]; V.ny = n[1]; V.nz = n[2];
             V.ax = L.frac[0]; V.ay = L.frac[1]; V.az = L.frac[2]; V.fyc = L.fyc;
@@ -2653,11 +2709,11 @@ wp_status build_hierarchy(wp_mgfrac3d* h, const float* ax, const float* ay, cons
             const float dmin = ((mn[1] + mn[0]) + zlo[zr]) + zlo[n[2] + zr];
             L.fz_fast = dmin > 1e-10f ? 1 : 0;
         }
-        WP_CUDA_TRY(cudaMalloc((void**)&L.tab64, sizeof(double) * t64.size()));
-        WP_CUDA_TRY(cudaMalloc((void**)&L.tab32, sizeof(float) * t32.size()));
+        WP_CUDA_TRY(h->mem.get(&L.tab64, sizeof(double) * t64.size()));
+        WP_CUDA_TRY(h->mem.get(&L.tab32, sizeof(float) * t32.size()));
         WP_CUDA_TRY(cudaMemcpy(L.tab64, t64.data(), sizeof(double) * t64.size(), cudaMemcpyHostToDevice));
         WP_CUDA_TRY(cudaMemcpy(L.tab32, t32.data(), sizeof(float) * t32.size(), cudaMemcpyHostToDevice));
-        WP_CUDA_TRY(cudaMalloc((void**)&L.uni, (size_t)n[0] * n[2]));
+        WP_CUDA_TRY(h->mem.get(&L.uni, (size_t)n[0] * n[2]));
         WP_KERNEL("uniform_rows", 16.0 * L.cells, s,
                   uniform_rows_kernel<<<std::min<unsigned>(wp_cdiv((long)n[0] * n[2] * 32, 256), 4096), 256, 0, s>>>(
                       L.uni, L.frac[0], L.fyc, L.frac[2], n[0], n[1], n[2], view<double>(L).glo[2], view<double>(L).ghi[2]));
@@ -2668,21 +2724,16 @@ wp_status build_hierarchy(wp_mgfrac3d* h, const float* ax, const float* ay, cons
             L.uni_rows = 0;
             for (unsigned char b : u) L.uni_rows += b != 0;
         }
-        WP_CUDA_TRY(cudaMalloc((void**)&L.v, sizeof(float) * L.cells));
-        WP_CUDA_TRY(cudaMalloc((void**)&L.t, sizeof(float) * L.cells));
-        WP_CUDA_TRY(cudaMalloc((void**)&L.f, sizeof(float) * L.cells));
+        for (float** p : {&L.v, &L.t, &L.f}) WP_CUDA_TRY(h->mem.get(p, sizeof(float) * L.cells));
         WP_CUDA_TRY(cudaMemsetAsync(L.v, 0, sizeof(float) * L.cells, s));
-        ++nl;
-        // next level: ceil halving, coarse spacing = sum of the two fine spacings (cuRestrictDx)
+        // next level: coarse spacing = sum of the two fine spacings (cuRestrictDx)
         for (int a = 0; a < dims; ++a) {
             const int m = wp_half_up(n[a]);
             std::vector<double> c(m);
             for (int i = 0; i < m; ++i) c[i] = hd[a][2 * i] + (2 * i + 1 < n[a] ? hd[a][2 * i + 1] : 0.0);
             hd[a] = c;
-            n[a] = m;
         }
     }
-    h->nl = nl;
     return WP_OK;
 }
 
@@ -2732,7 +2783,7 @@ bool cluster_placed(const CyPack& pack, bool d2, cudaStream_t s) {
 void choose_pack(wp_mgfrac3d* h, CyPlan* q, int most) {
     const bool d2 = h->dims == 2;
     q->l0 = h->nl;
-    for (int l = 0; l + 2 <= h->nl; ++l) {
+    for (int l = 0; most > 0 && l + 2 <= h->nl; ++l) {
         int e[kMaxLevels][3];
         for (int k = l; k < h->nl; ++k) {
             const int* n = h->lv[k].n;
@@ -2757,7 +2808,7 @@ wp_status build_cycle_plan(wp_mgfrac3d* h, CyPlan* q, int most, cudaStream_t s) 
         q->l0 = h->nl;
     }
     if (q->l0 == h->nl) return WP_OK;
-    WP_CUDA_TRY(cudaMalloc((void**)&q->image, sizeof(float) * (size_t)q->pack.image * q->pack.ctas));
+    WP_CUDA_TRY(h->mem.get(&q->image, sizeof(float) * (size_t)q->pack.image * q->pack.ctas));
     WP_CUDA_TRY(cudaMemsetAsync(q->image, 0, sizeof(float) * (size_t)q->pack.image * q->pack.ctas, s));
     for (int k = 0; k < q->pack.n; ++k) {
         const Level& L = h->lv[q->l0 + k];
@@ -3253,13 +3304,10 @@ wp_status defect(wp_mgfrac3d* h, const TP* p, const float* f, double m, float* r
 void destroy_levels(wp_mgfrac3d* h) {
     for (int l = 0; l < kMaxLevels; ++l) {
         Level& L = h->lv[l];
-        for (int a = 0; a < 3; ++a) if (L.frac[a]) cudaFree(L.frac[a]);
-        void* ps[] = {L.tab64, L.tab32, L.fyc, L.uni, L.tuni, L.v, L.t, L.f, L.v64, L.t64, L.f64, L.imask, L.iseg};
+        void* ps[] = {L.v64, L.t64, L.f64, L.imask, L.iseg};
         for (void* p : ps) if (p) cudaFree(p);
     }
-    for (CyPlan* q : {&h->cy, &h->one})
-        if (q->image) cudaFree(q->image);
-    if (h->acc) cudaFree(h->acc);
+    h->mem.free();
     if (h->p64) cudaFree(h->p64);
     if (h->r32) cudaFree(h->r32);
     if (h->ix_r) cudaFree(h->ix_r);
@@ -3282,11 +3330,12 @@ wp_status create_common(wp_mgfrac3d** out, int dims, const float* ax, const floa
     h->coarsest_iters = dims == 3 ? 50 : 10;
     h->mid_on = 0;
     h->fz_on = 1;
+    const int limit = g_cluster_limit.exchange(-1), most = limit < 0 ? 16 : std::min(limit, 16), ext[3] = {nx, ny, nz};
+    size_levels(h, ext, most);
     wp_status st = build_hierarchy(h, ax, ay, az, nx, ny, nz, dx, dy, dz, s);
-    const int limit = g_cluster_limit.exchange(-1);
-    if (st == WP_OK) st = build_cycle_plan(h, &h->cy, limit < 0 ? 16 : std::min(limit, 16), s);
+    if (st == WP_OK) st = build_cycle_plan(h, &h->cy, most, s);
     if (st == WP_OK) {
-        cudaError_t e = cudaMalloc((void**)&h->acc, 4 * sizeof(double) + 16);
+        cudaError_t e = h->mem.get(&h->acc, 4 * sizeof(double) + 16);
         // the int error flag lives in the 16 bytes after the four FP64 slots
         if (e == cudaSuccess) e = cudaMemsetAsync(h->acc, 0, 4 * sizeof(double) + 16, s);
         if (e == cudaSuccess)
