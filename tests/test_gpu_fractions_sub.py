@@ -79,3 +79,19 @@ def test_non_finite_level_sets_match_oracle(wp, oracle):
     for r, o in zip(oracle.fractions3d_subsampled(ls.astype(np.float64), n, h), _frac(wp, ls, n, h)):
         assert np.array_equal(o, r)
         assert (r == 0).any() and (r == 1).any()
+
+
+@pytest.mark.parametrize("far", [1e8, 1e30, 3e38])
+@pytest.mark.parametrize("h", [0.3, 1e-20])
+def test_huge_values_classify_as_in_fp64(wp, far, h):
+    """Cells marked by a huge value: where positions round, taps of nominal weight 0 count.  The same cells beside one that is
+    not a number, which makes every face take FP64, give the same fractions (bound 0) away from it."""
+    n = (24, 17, 16)
+    rng = np.random.default_rng(8)
+    ls = (rng.standard_normal((n[2], n[0], n[1])) * 4 * h).astype(np.float32)
+    ls.reshape(-1)[::503] = far
+    fp64 = ls.copy()
+    fp64[:, -1] = np.nan
+    for a, b in zip(_frac(wp, ls, n, h), _frac(wp, fp64, n, h)):
+        assert np.array_equal(a[:, :20], b[:, :20])
+        assert 0.1 < (a[:, :20] > 0).mean() < 0.9

@@ -504,22 +504,31 @@ __device__ __forceinline__ float face_quadratic32(const float* __restrict__ ls, 
     return r;
 }
 
-// *flag = 1 when ls holds a value that is not finite
-__global__ void __launch_bounds__(256) nonfinite_kernel(const float* __restrict__ ls, long n, unsigned* __restrict__ flag) {
-    bool bad = false;
-    for (long i = blockIdx.x * 256L + threadIdx.x; i < n; i += 256L * gridDim.x) bad |= !isfinite(ls[i]);
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) *flag = 1;
+// *most = the largest |value| of ls as bits (from 0x7f800000 on: it holds one that is not finite)
+__global__ void __launch_bounds__(256) magnitude_kernel(const float* __restrict__ ls, long n, unsigned* __restrict__ most) {
+    unsigned m = 0;
+    for (long i = blockIdx.x * 256L + threadIdx.x; i < n; i += 256L * gridDim.x) m = max(m, __float_as_uint(ls[i]) & 0x7fffffffu);
+    m = __reduce_max_sync(0xffffffffu, m);
+    __shared__ unsigned red[8];
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) m = max(m, red[k]);
+        if (m > *(volatile unsigned*)most) atomicMax(most, m);
+    }
 }
 
 // Open, closed or cut, by the quadratic interpolant at the face centre against +-dx.  The FP64 interpolant
 // (27 taps) was the cost: 130 us for 6 M faces of a 160 x 128 x 97 grid, 20 x its
 // 25 MB (now 70, and 5 for the test of the values).  The FP32 one is
 // off by at most 21 roundings of the largest value read (a convex combination), so it decides wherever
-// it is further than 4e-6 of that value from both thresholds; the rest take FP64.  A level set with a value
-// that is not finite takes FP64 throughout: its 27 taps include some of weight 0 that are not read here.
+// it is further than 4e-6 of that value from both thresholds; the rest take FP64.  The FP64 one's 27 taps include
+// some that are not read here: at a position rounded off by d cells (8 eps64 times the largest extent at most) they
+// weigh d^2 / 2, so that d^2 (far) of the largest value anywhere joins the margin.  A level set with a value
+// that is not finite takes FP64 throughout.
 __global__ void __launch_bounds__(256) frac_classify_kernel(float* __restrict__ ax, float* __restrict__ ay,
                                                             float* __restrict__ az, const float* __restrict__ ls,
-                                                            int nx, int ny, int nz, double dx,
+                                                            int nx, int ny, int nz, double dx, double far,
                                                             unsigned* __restrict__ work, unsigned* __restrict__ nwork) {
     // blockIdx.z: the axis; a warp walks 32 consecutive faces along y
     const int a = blockIdx.z;
@@ -528,7 +537,9 @@ __global__ void __launch_bounds__(256) frac_classify_kernel(float* __restrict__ 
     const unsigned segs = (unsigned)nrow * ex * ez;  // fewer than 2^30 faces
     float* out = a == 0 ? ax : (a == 1 ? ay : az);
     const float d32 = (float)dx;
-    const bool all64 = nwork[1] != 0;  // set by nonfinite_kernel
+    const unsigned most = nwork[1];  // by magnitude_kernel
+    const bool all64 = most >= 0x7f800000u;
+    const float beyond = (float)(far * (double)__uint_as_float(most));
     for (unsigned sgm = blockIdx.x * 8u + (threadIdx.x >> 5); sgm < segs; sgm += gridDim.x * 8u) {
         const unsigned row = sgm / (unsigned)nrow, z = row / (unsigned)ex, x = row - z * ex;
         const int y = (int)(sgm - row * nrow) * 32 + lane;
@@ -537,7 +548,7 @@ __global__ void __launch_bounds__(256) frac_classify_kernel(float* __restrict__ 
         if (y < ey) {
             float big;
             const float v32 = face_quadratic32(ls, a, x, y, z, nx, ny, nz, &big);
-            const float margin = 4e-6f * (big + d32);
+            const float margin = 4e-6f * (big + d32) + beyond;
             bool open = !all64 && v32 > d32 + margin;
             cut = !all64 && fabsf(v32) < d32 - margin;
             if (all64 || (!open && !cut && !(v32 < -d32 - margin))) {
@@ -651,20 +662,21 @@ extern "C" CUWHHD_API wp_status wp_fractions3d_subsampled(float* ax, float* ay, 
     const long faces = (long)(nx + 1) * ny * nz + (long)nx * (ny + 1) * nz + (long)nx * ny * (nz + 1);
     unsigned* buf = nullptr;
     WP_CUDA_TRY(wp_scratch_alloc((void**)&buf, sizeof(unsigned) * (faces + 2), s));
-    // buf: the number of cut faces, the flag of a value that is not finite, the list
+    // buf: the number of cut faces, the largest |value|, the list
     cudaError_t e = cudaMemsetAsync(buf, 0, 2 * sizeof(unsigned), s);
     if (e == cudaSuccess) {
         const int tok = wp_prof_start(s);
         const long cells = (long)nx * ny * nz;
-        nonfinite_kernel<<<(unsigned)std::min<long>(wp_cdiv(cells, 1024), (long)wp_sm_count() * 8), 256, 0, s>>>(ls, cells,
+        magnitude_kernel<<<(unsigned)std::min<long>(wp_cdiv(cells, 1024), (long)wp_sm_count() * 8), 256, 0, s>>>(ls, cells,
                                                                                                             buf + 1);
         e = cudaGetLastError();
-        wp_prof_stop(tok, "frac_nonfinite", 4.0 * cells, s);
+        wp_prof_stop(tok, "frac_magnitude", 4.0 * cells, s);
     }
     if (e == cudaSuccess) {
         const int tok = wp_prof_start(s);
         const dim3 g((unsigned)std::min<long>(wp_cdiv(faces, 3 * 256), (long)wp_sm_count() * 8), 1, 3);
-        frac_classify_kernel<<<g, 256, 0, s>>>(ax, ay, az, ls, nx, ny, nz, dx, buf + 2, buf);
+        const double d = 8.0 * 2.2e-16 * std::max(nx, std::max(ny, nz));
+        frac_classify_kernel<<<g, 256, 0, s>>>(ax, ay, az, ls, nx, ny, nz, dx, d * d, buf + 2, buf);
         e = cudaGetLastError();
         wp_prof_stop(tok, "frac_classify", 4.0 * faces + 4.0 * nx * ny * nz, s);
     }
