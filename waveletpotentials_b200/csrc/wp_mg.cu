@@ -109,8 +109,10 @@ __device__ __forceinline__ T cell_diag(const Lvl<T>& L, int x, int y, int z) {
 // z-face fraction carried in registers, so each v and az value of the column is loaded once; in-plane
 // neighbours come through L1 (they are loaded by the neighbouring threads of the CTA).  A step gives the
 // swept value (SWEEP) or the residual, 0 where the cell is inactive.
-// LEAN: rows flagged kUniLean read no fractions and divide by nothing.  201 x 150 x 101: a finest sweep 29.8 -> 21
-// us, the restriction 37 -> 22.5, the FP64 defect 55 -> 36 (1.9 TB/s of L2 and DRAM traffic, latency of the column).
+// LEAN: rows flagged kUniLean read no fractions and divide by nothing.  201 x 150 x 101, FP32: a finest sweep 30.4 -> 23.0
+// us, the restriction 36.9 -> 23.4 (FP64 55.7 -> 36.9).  FP64 sweeps and the defect do without: a division
+// ahead of every chunk and the second path cost more than they save (201 x 150 x 101: 36.5 -> 35.5 and
+// 47.7 -> 38.2 us; 100 x 101 x 102: 22.9 -> 20.8 and 30.7 -> 24.5); rows of open faces read no fractions in either form.
 // Without it the operations are QCol's: where a level of whole quads could run either kernel (by the tuner's choice or
 // an argument's alignment), its one-cell kernel takes that form, so that the choice never shows in the bits.
 template <typename T, typename TV, bool PROL, bool SWEEP, bool LEAN>
@@ -1852,7 +1854,7 @@ __global__ void __launch_bounds__(256) defect64_kernel(float* __restrict__ r32, 
 // walls the operator's null space is the constant on the active cells, so a right-hand side stored
 // in FP32 carries an incompatible constant part of FP32 rounding size that floors the residual
 // (about 2e-10 relative at 64^3); the tolerance-driven solve removes that mean in FP64.
-template <typename TP, bool LEAN>
+template <typename TP>
 __global__ void __launch_bounds__(256) defect64_z_kernel(float* __restrict__ r32, const TP* __restrict__ p,
                                                          const float* __restrict__ f, Lvl<double> L, double m,
                                                          const double* __restrict__ msum, double* __restrict__ acc,
@@ -1863,7 +1865,7 @@ __global__ void __launch_bounds__(256) defect64_z_kernel(float* __restrict__ r32
     if (msum) m = msum[0] / fmax(msum[1], 1.0);  // mean of f over the active cells, computed on the device
     double s2 = 0.0;
     if (y < L.ny && x < L.nx && z0 < z1) {
-        ZCol<double, TP, false, false, LEAN> col(L, p, nullptr, 0, 0, x, y, z0);
+        ZCol<double, TP, false, false, false> col(L, p, nullptr, 0, 0, x, y, z0);
         for (int z = z0; z < z1; ++z) {
             const long i = col.i;
             const double r = col.step((double)f[i] - m);
@@ -2361,7 +2363,7 @@ void launch_jacobi(const Level& L, T* dst, const T* src, const T* f, T w, int zc
         else if (var == 2) wp_launch_pdl(jacobi_q_mb_kernel<T, 4>, g, 256, 0, s, dst, src, f, V, w, zc, nullptr);
         else wp_launch_pdl(jacobi_q_kernel<T>, g, 256, 0, s, dst, src, f, V, w, zc, nullptr);
     } else {
-        wp_launch_pdl(quad_ok(L) ? jacobi_z_kernel<T, false, false> : jacobi_z_kernel<T, false, true>,
+        wp_launch_pdl(sizeof(T) == 8 || quad_ok(L) ? jacobi_z_kernel<T, false, false> : jacobi_z_kernel<T, false, true>,
                       grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, dst, src, f, V, w, (const T*)nullptr, 0, 0, zc,
                       (double*)nullptr);
     }
@@ -2444,8 +2446,8 @@ void launch_defect64(const Level& L, float* r32, const TP* p, const float* f, do
         }
         wp_launch_pdl(defect64_q_kernel<TP>, g, 256, 0, s, r32, p, f, V, m, msum, acc, zc);
     } else {
-        wp_launch_pdl(quad_ok(L) ? defect64_z_kernel<TP, false> : defect64_z_kernel<TP, true>,
-                      grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, r32, p, f, V, m, msum, acc, zc);
+        wp_launch_pdl(defect64_z_kernel<TP>, grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, r32, p, f, V, m, msum,
+                      acc, zc);
     }
 }
 
@@ -3169,7 +3171,7 @@ wp_status vcycle(wp_mgfrac3d* h, int l, const T* f, int nu1, int nu2, T w, int p
             // first post-sweep reads v + P vc directly (prolongation fused into the sweep)
             const int zc = level_zc(L, kZcJacobi);
             WP_KERNEL("jacobi_prolong", (double)L.cells * (3.0 * sizeof(T) + 12.0) + (double)C.cells * sizeof(T), s,
-                      jacobi_z_kernel<T, true, true><<<grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s>>>(
+                      jacobi_z_kernel<T, true, sizeof(T) == 4><<<grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s>>>(
                           Bufs<T>::t(L), Bufs<T>::v(L), f, view<T>(L), w, Bufs<T>::v(C), C.n[0], C.n[1], zc));
             T* tmp = Bufs<T>::v(L);
             Bufs<T>::v(L) = Bufs<T>::t(L);
