@@ -13,7 +13,8 @@ def T(a):
     return torch.as_tensor(np.ascontiguousarray(a), dtype=torch.float32, device="cuda")
 
 
-def _problem(oracle, n, seed):
+def _problem(oracle, n, seed, steps=0):
+    """steps: fractions in 1 / steps (a power of two), which every level's averages of them hold exactly"""
     rng = np.random.default_rng(seed)
     dims = len(n)
     h = 1.0 / max(n)
@@ -25,7 +26,7 @@ def _problem(oracle, n, seed):
         x, y = np.meshgrid((np.arange(n[0]) + 0.5) * h, (np.arange(n[1]) + 0.5) * h, indexing="ij")
         a = oracle.fractions2d(np.hypot(x - 0.4 * n[0] * h, y - 0.5 * n[1] * h) - 0.2 * min(n) * h, n, h)
         cells, ax = tuple(n), (0, 1)
-    a = [v.astype(np.float32).astype(np.float64) for v in a]
+    a = [np.round(v * steps) / steps if steps else v.astype(np.float32).astype(np.float64) for v in a]
     diag = np.zeros(cells)
     for v, d in zip(a, ax):
         m = v.shape[d] - 1
