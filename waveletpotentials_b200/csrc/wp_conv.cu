@@ -232,7 +232,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // 16-byte cp.async from four producer warps (zero-filled outside the volume).  Two accumulators in TMEM: the
 // epilogue of a plane overlaps the next plane's products.
 // What bounds it is the rate of the products, some 140 cycles each of 128 x N x 16 whatever N is.  Measured at
-// 64^3 (B200): 16 -> 16 channels 70 -> 32 us, 32 -> 32 78 -> 60, 16 + 32 -> 16 123 -> 79; at 32^3 and 16^3 within
+// 64^3 (B200): 16 -> 16 channels 70 -> 32 us, 32 -> 32 78 -> 62, 16 + 32 -> 16 123 -> 80; at 32^3 and 16^3 within
 // 2 us of conv3_fwd_kernel, mostly below it.
 struct WalkGeo {
     int pitch;     // ny + 2

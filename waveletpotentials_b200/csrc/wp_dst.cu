@@ -216,8 +216,8 @@ cudaError_t launch_axis(const double* src, double* dst, const double* M, int n, 
     return e;
 }
 
-// 32 lines and 8 warps up to 256 (74 KB of shared memory: three CTAs per SM, whose loads and products
-// overlap); longer lines take 16 columns so that the tile and the accumulators still fit (82 KB at 512,
+// 32 lines and 8 warps up to 256 (74 KB of shared memory and some 120 registers: two CTAs per SM, whose loads and
+// products overlap); longer lines take 16 columns so that the tile and the accumulators still fit (82 KB at 512,
 // 164 KB at 1024).
 template <int MODE>
 cudaError_t launch_mode(const double* src, double* dst, const double* M, int n, Geom g, int nx, int ny, double scale,

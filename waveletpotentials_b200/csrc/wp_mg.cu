@@ -1443,7 +1443,8 @@ __global__ void __launch_bounds__(256) prolong_tri_z_kernel(T* __restrict__ v, c
 }
 
 // ------------------------------------------------------------------ fused coarse cycle
-// The V-cycle below a small level (<= kCoarseCells cells) in ONE single-CTA launch: zeroing, sweeps,
+// FP64 cycles, and FP32 levels outside a pack (wp_mg_cluster.cuh): the V-cycle below a small level (<= kCoarseCells
+// cells) in ONE single-CTA launch: zeroing, sweeps,
 // residual restriction, coarsest sweeps and prolongation of every coarse level, with block barriers
 // between the steps (the data stay in L2).  At these sizes every separate kernel is a few
 // microseconds of launch and ramp for a few thousand cells.  Per cell the arithmetic is that of the
