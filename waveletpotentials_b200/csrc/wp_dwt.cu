@@ -1192,12 +1192,17 @@ cudaError_t launch_lines(const LineJobs& jobs, int n, bool contig, bool fwd, cud
                        : launch_line_k<T, false, MOVE, P0, MAXT, MINB>(jobs, grid, nt, smem, s);
         };
         if (!contig) return dir(std::integral_constant<int, LM_STRIDED>());
-        if (N < kLineRun) return dir(std::integral_constant<int, LM_RUN>());
+        if constexpr (sizeof(T) == 8 || MAXT == 256)
+            if (N < kLineRun) return dir(std::integral_constant<int, LM_RUN>());
         return dir(std::integral_constant<int, LM_LINES>());
     };
     cudaError_t e;
-    if (sizeof(T) == 4 && nt <= 256) e = go(std::integral_constant<int, 256>(), std::integral_constant<int, 3>());
-    else e = go(std::integral_constant<int, 512>(), std::integral_constant<int, 1>());
+    const std::integral_constant<int, 512> m512;
+    const std::integral_constant<int, 1> m1;
+    if constexpr (sizeof(T) == 4)
+        e = nt <= 256 ? go(std::integral_constant<int, 256>(), std::integral_constant<int, 3>()) : go(m512, m1);
+    else
+        e = go(m512, m1);
     wp_prof_stop(tok, fwd ? "dwt_forward" : "dwt_inverse", bytes, s);
     return e;
 }

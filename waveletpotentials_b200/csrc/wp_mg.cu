@@ -2364,7 +2364,7 @@ void launch_jacobi(const Level& L, T* dst, const T* src, const T* f, T w, int zc
         else if (var == 2) wp_launch_pdl(jacobi_q_mb_kernel<T, 4>, g, 256, 0, s, dst, src, f, V, w, zc, nullptr);
         else wp_launch_pdl(jacobi_q_kernel<T>, g, 256, 0, s, dst, src, f, V, w, zc, nullptr);
     } else {
-        wp_launch_pdl(sizeof(T) == 8 || quad_ok(L) ? jacobi_z_kernel<T, false, false> : jacobi_z_kernel<T, false, true>,
+        wp_launch_pdl(quad_ok(L) ? jacobi_z_kernel<T, false, false> : jacobi_z_kernel<T, false, sizeof(T) == 4>,
                       grid_z(L.n[0], L.n[1], L.n[2], zc), dim3(32, 8), 0, s, dst, src, f, V, w, (const T*)nullptr, 0, 0, zc,
                       (double*)nullptr);
     }
