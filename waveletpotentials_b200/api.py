@@ -941,13 +941,13 @@ class BatchProjector:
             pass
 
 
-# ------------------------------------------------------------------ test-only failure injection
 def release_scratch():
     """Gives the device memory that the level-set calls keep between them (at most 64 MB per device) back
     to the driver (wp_release_scratch)."""
     check(lib().wp_release_scratch(), "wp_release_scratch")
 
 
+# ------------------------------------------------------------------ test-only hooks
 def debug_cluster_limit(ctas):
     """Test-only: the next multigrid handle is created as on a device that places thread-block clusters of
     at most ``ctas`` CTAs (wp_debug_cluster_limit).  One shot."""
